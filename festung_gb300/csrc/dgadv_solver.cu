@@ -74,6 +74,24 @@ static uint32_t morton2(uint32_t x, uint32_t y) {
   return spread(x) | (spread(y) << 1);
 }
 
+// Within each block of kBlock elements: elements whose first edge faces the same way next to each
+// other (eight sectors centred on the axes and diagonals; Morton order within a sector).  Which of
+// its edges an element takes inflow through follows from their directions against the velocity,
+// which hardly varies over a block; so the lanes of a warp then take the same branches of the
+// upwind flux, where the two orientations of a triangulated grid otherwise alternate and every
+// warp runs the terms of both.  The block as a whole, and so its locality, stays the same.
+static void group_by_orientation(const Grid &gr, const std::vector<int> &instStart, std::vector<int> &perm) {
+  std::vector<uint8_t> sector(perm.size());
+  for (size_t t = 0; t < perm.size(); ++t) {
+    const double a = std::atan2(gr.nuE0T[6 * t + 1], gr.nuE0T[6 * t]) * (4.0 / 3.14159265358979323846);
+    sector[t] = (uint8_t)((int)std::floor(a + 0.5) & 7);
+  }
+  for (size_t i = 0; i + 1 < instStart.size(); ++i)
+    for (int b = instStart[i]; b < instStart[i + 1]; b += kBlock)
+      std::stable_sort(perm.begin() + b, perm.begin() + std::min(b + kBlock, instStart[i + 1]),
+                       [&](int x, int y) { return sector[x] < sector[y]; });
+}
+
 // One handle over one mesh, or over the disjoint union of an ensemble's meshes: instStart holds
 // the first element of every instance and the total element count (empty: one instance).
 static int create_impl(const dgadv_mesh *mesh, const dgadv_params *prm, const std::vector<int> &instStart,
@@ -145,6 +163,7 @@ static int create_impl(const dgadv_mesh *mesh, const dgadv_params *prm, const st
         key[t] = morton2((uint32_t)((gr.baryT[2 * t] - xmin) * sx), (uint32_t)((gr.baryT[2 * t + 1] - ymin) * sy));
       std::stable_sort(perm.begin() + t0, perm.begin() + t1, [&](int a, int b) { return key[a] < key[b]; });
     }
+    group_by_orientation(gr, h->instStart, perm);
   }
   std::vector<int> inv(K);
   for (int k = 0; k < K; ++k) inv[perm[k]] = k;
