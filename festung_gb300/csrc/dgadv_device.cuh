@@ -28,6 +28,7 @@
 #include "dgadv_handle.h"
 #include "dgadv_kernels.cuh"
 #include "dgadv_df32.cuh"
+#include "dgadv_fixed.cuh"
 
 namespace dgadv {
 
@@ -35,6 +36,7 @@ namespace dgadv {
 template <typename T, int P> __device__ __forceinline__ const Tab<T, P> &tab();
 namespace {
 template <typename T, int P> const void *tab_symbol();   // host address of the unit's table
+template <int P> const void *fx_symbol();                // ... of the FP64 unit's digit tables
 }  // namespace
 
 #define DGADV_DEFINE_TABLES(T, NAME)                                                            \
@@ -51,6 +53,23 @@ template <typename T, int P> const void *tab_symbol();   // host address of the 
   template <> [[maybe_unused]] const void *tab_symbol<T, 1>() { return (const void *)&NAME##1; }  \
   template <> [[maybe_unused]] const void *tab_symbol<T, 2>() { return (const void *)&NAME##2; }  \
   template <> [[maybe_unused]] const void *tab_symbol<T, 3>() { return (const void *)&NAME##3; }  \
+  }
+
+// The digit tables of the FP64 units (dgadv_fixed.cuh).
+#define DGADV_DEFINE_DIGIT_TABLES(NAME)                                                         \
+  static __constant__ FxTab<0> NAME##0;                                                         \
+  static __constant__ FxTab<1> NAME##1;                                                         \
+  static __constant__ FxTab<2> NAME##2;                                                         \
+  static __constant__ FxTab<3> NAME##3;                                                         \
+  template <> __device__ __forceinline__ const FxTab<0> &fx_tab<0>() { return NAME##0; }        \
+  template <> __device__ __forceinline__ const FxTab<1> &fx_tab<1>() { return NAME##1; }        \
+  template <> __device__ __forceinline__ const FxTab<2> &fx_tab<2>() { return NAME##2; }        \
+  template <> __device__ __forceinline__ const FxTab<3> &fx_tab<3>() { return NAME##3; }        \
+  namespace {                                                                                   \
+  template <> [[maybe_unused]] const void *fx_symbol<0>() { return (const void *)&NAME##0; }    \
+  template <> [[maybe_unused]] const void *fx_symbol<1>() { return (const void *)&NAME##1; }    \
+  template <> [[maybe_unused]] const void *fx_symbol<2>() { return (const void *)&NAME##2; }    \
+  template <> [[maybe_unused]] const void *fx_symbol<3>() { return (const void *)&NAME##3; }    \
   }
 
 // ---------------------------------------------------------------------------------------------
@@ -77,7 +96,7 @@ template <typename T> __host__ __device__ constexpr unsigned long long key_max()
 template <> __host__ __device__ constexpr unsigned long long key_max<double>() { return ~0ULL; }
 template <> __host__ __device__ constexpr unsigned long long key_max<float>() { return 0xFFFFFFFFULL; }
 
-__device__ __forceinline__ bool finite_(double x) { return isfinite(x); }
+__device__ __forceinline__ bool finite_(double x) { return fx::finite_bits(x); }   // no FP64 comparison
 __device__ __forceinline__ bool finite_(float x) { return isfinite(x); }
 
 // df32: the key of hi in the high half and the key of lo in the low half orders pairs like
@@ -392,6 +411,24 @@ __device__ __forceinline__ size_t slot_base(const Geo<T> &g, int nc, int tile = 
   return g.instOf ? (size_t)g.instOf[(tile * (int)blockDim.x) / kBlock] * kSlotCopies * 2 * nc : 0;
 }
 
+// Least / greatest of a warp's 32-bit or 64-bit keys (the low words among the lanes that hold the
+// extreme high word).
+__device__ __forceinline__ unsigned int warp_min(unsigned int k) { return __reduce_min_sync(0xffffffffu, k); }
+__device__ __forceinline__ unsigned int warp_max(unsigned int k) { return __reduce_max_sync(0xffffffffu, k); }
+__device__ __forceinline__ unsigned long long warp_min(unsigned long long k) {
+  const unsigned int h = (unsigned int)(k >> 32), m = warp_min(h);
+  return ((unsigned long long)m << 32) | warp_min(h == m ? (unsigned int)k : 0xffffffffu);
+}
+__device__ __forceinline__ unsigned long long warp_max(unsigned long long k) {
+  const unsigned int h = (unsigned int)(k >> 32), m = warp_max(h);
+  return ((unsigned long long)m << 32) | warp_max(h == m ? (unsigned int)k : 0u);
+}
+__device__ __forceinline__ bool nan_(float x) { return x != x; }
+__device__ __forceinline__ bool nan_(double x) {
+  return ((unsigned long long)__double_as_longlong(x) << 1) > 0xFFE0000000000000ULL;
+}
+__device__ __forceinline__ bool nan_(const df32 &x) { return x.hi != x.hi || x.lo != x.lo; }
+
 // Scatter of the element's centroid quantities to its vertices and the block's global extremes.
 template <typename T, int NQ>
 __device__ __forceinline__ void scatter_quantities(const Geo<T> &g, const LimOut<T> &lo, const T *qv,
@@ -409,30 +446,30 @@ __device__ __forceinline__ void scatter_quantities(const Geo<T> &g, const LimOut
       }
     }
   }
-  // global extremes: warp shuffles, then the block's four warps through shared memory, then one
-  // atomic per quantity and block into one of kSlotCopies copies (spreads same-address atomics)
-  __shared__ T red[kBlock / 32][2 * NQ];
+  // global extremes of the ordered keys (min and max of integers: no FP64 comparisons), by one
+  // redux per 32 bits and warp, then the block's warps through shared memory, then one atomic per
+  // quantity and block into one of kSlotCopies copies (spreads same-address atomics).  A NaN takes no
+  // part, as fmin / fmax ignore it.
+  using K_ = typename KeyOf<T>::type;
+  __shared__ K_ red[kBlock / 32][2 * NQ];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 #pragma unroll
   for (int s = 0; s < NQ; ++s) {
-    T mn = (active && s < lo.nc) ? qv[s] : T(INFINITY), mx = (active && s < lo.nc) ? qv[s] : T(-INFINITY);
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      mn = fmin(mn, __shfl_xor_sync(0xffffffffu, mn, o));
-      mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-    }
+    const bool in = active && s < lo.nc && !nan_(qv[s]);
+    const K_ key = in ? vkey(qv[s]) : K_(0);
+    const K_ mn = warp_min(in ? key : vkey_max<T>()), mx = warp_max(key);
     if (lane == 0) { red[warp][2 * s] = mn; red[warp][2 * s + 1] = mx; }
   }
   __syncthreads();
   if (threadIdx.x < lo.nc) {
     const int s = threadIdx.x;
-    T mn = red[0][2 * s], mx = red[0][2 * s + 1];
+    K_ mn = red[0][2 * s], mx = red[0][2 * s + 1];
 #pragma unroll
-    for (int w = 1; w < (int)(blockDim.x / 32); ++w) { mn = fmin(mn, red[w][2 * s]); mx = fmax(mx, red[w][2 * s + 1]); }
+    for (int w = 1; w < (int)(blockDim.x / 32); ++w) { mn = min(mn, red[w][2 * s]); mx = max(mx, red[w][2 * s + 1]); }
     if (mn <= mx) {
       unsigned long long *sl = lo.slots + slot_base(g, lo.nc, tile) + (size_t)(tile % kSlotCopies) * 2 * lo.nc;
-      atomicMin(&sl[2 * s], okey(mn));
-      atomicMax(&sl[2 * s + 1], okey(mx));
+      atomicMin(&sl[2 * s], (unsigned long long)mn);
+      atomicMax(&sl[2 * s + 1], (unsigned long long)mx);
     }
   }
 }
@@ -460,14 +497,10 @@ template <typename T>
 __device__ __forceinline__ void load_shifts(const unsigned long long *slots, int nc, T *sh) {
   if (threadIdx.x >= 32) return;
   const int lane = threadIdx.x;
+  using K_ = typename KeyOf<T>::type;
   for (int s = 0; s < nc; ++s) {
-    T mn = okey_inv<T>(slots[(size_t)lane * 2 * nc + 2 * s]);
-    T mx = okey_inv<T>(slots[(size_t)lane * 2 * nc + 2 * s + 1]);
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      mn = fmin(mn, __shfl_xor_sync(0xffffffffu, mn, o));
-      mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-    }
+    const T mn = okey_inv<T>(warp_min((K_)slots[(size_t)lane * 2 * nc + 2 * s]));
+    const T mx = okey_inv<T>(warp_max((K_)slots[(size_t)lane * 2 * nc + 2 * s + 1]));
     if (lane == 0) { sh[2 * s] = fabs(mn) + T(1); sh[2 * s + 1] = fabs(mx) + T(1); }
   }
 }
@@ -582,7 +615,9 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint64_t *bar, int *flag) {
   return true;
 }
 
-// Row copies into the staged layout (row index within the T rows / the int rows).
+// Row copies into the staged layout (row index within the T rows / the int rows), by one thread: the
+// instruction takes uniform registers, so lanes issuing rows side by side become a loop over the
+// lanes (measured: 524288 triangles, p = 3, hierarchical limiter 4 % slower).
 template <typename T>
 __device__ __forceinline__ void stage_T(unsigned char *smem, int row, const T *base, int nrows, int Kp, int k0,
                                         uint64_t *bar) {
@@ -934,12 +969,14 @@ struct StageScalars {
 //   kOpFp32     (double-float state only) the operator (volume, flux, hatM^-1 = I) in FP32
 //               arithmetic; the SSP update, the outputs and the limiter's quantities stay in the
 //               stored type;
-//   kOpElement  (FP64 or double-float, no source terms) the element operator g.Aop, N x N per element: the
-//               volume term and the element's own outflow terms as one product with c, built
-//               by k_build_element_operator whenever the velocity changes; only the inflow terms
-//               are evaluated at the edge points.  GB300's FP64 rate bounds the FP64 stage: this
-//               takes the operator from about 244 FP64 instructions per element to about 100
-//               (p = 2).
+//   kOpElement  (FP64, or double-float without source terms) the element operator g.Aop, N x N per
+//               element: the volume term and the element's own outflow terms as one product with c,
+//               built by k_build_element_operator whenever the velocity changes; only the inflow
+//               terms are evaluated at the edge points, of neighbours that only inflow edges load.
+//               In FP64 the sums run in fixed point on the integer units (dgadv_fixed.cuh), since
+//               GB300's FP64 rate bounds them otherwise: 131072 triangles, p = 2, per launch (cold)
+//               51 -> 27 us, 2180 instructions per warp of which 20 in FP64 (about 190 before).
+//               Source terms are added in FP64, with hatM^-1 applied when they are set.
 constexpr int kOpPlain = 0, kOpFp32 = 1, kOpElement = 2;
 
 template <typename T, int P, int MODE, bool RHS, bool LIN, int VAR = kOpPlain>
@@ -947,6 +984,7 @@ __device__ __forceinline__ void stage_op_tile(const Geo<T> g, const T *cin, cons
            const LimOut<T> lo, const StageScalars sc, const int tile, const int nTiles = -1) {
   constexpr int N = Dims<P>::N, Q = Dims<P>::Q, R = Dims<P>::R, NQ = NCQ<P>::value;
   constexpr bool OPF = VAR == kOpFp32, EOP = VAR == kOpElement;
+  constexpr bool FXP = EOP && std::is_same_v<T, double>;   // the element operator in fixed point
   static_assert(!EOP || ((std::is_same_v<T, double> || std::is_same_v<T, df32>) && !RHS),
                 "the element operator is FP64 or double-float without source terms");
   using A = std::conditional_t<OPF, float, T>;
@@ -961,15 +999,21 @@ __device__ __forceinline__ void stage_op_tile(const Geo<T> g, const T *cin, cons
   pdl_trigger();
   const int Kp = g.Kp;
   const bool staged = k0 < g.K;                   // blocks beyond the elements only reset keys
+  const bool first = sc.omega == 0.0;             // c^n has no part in this stage: not read
   constexpr int rC = 0, rC0 = N, rF = (MODE != 2) ? 2 * N : N, rV = rF + (EOP ? N * N : 2 * Q), rB = rV + 3 * R;
   if (staged) {
     if (t == 0) { mbar_init(bar, 1); mbar_fence_init(); }
     __syncthreads();
     if (t == 0) {                                 // static rows before the dependency wait
-      stage_expect<T>(bar, NT, 1);
-      if constexpr (EOP) stage_T(smem, rF, g.Aop, N * N, Kp, k0, bar);
-      else stage_T(smem, rF, g.F, 2 * Q, Kp, k0, bar);
-      stage_T(smem, rV, g.Vn, 3 * R, Kp, k0, bar);
+      stage_expect<T>(bar, NT - (MODE != 2 && first ? N : 0), 1);
+      if constexpr (FXP) {       // digits: 8 bytes each, as the rows they stand for
+        stage_T(smem, rF, (const T *)g.AopX, N * N, Kp, k0, bar);
+        stage_T(smem, rV, (const T *)g.VnX, 3 * R, Kp, k0, bar);
+      } else {
+        if constexpr (EOP) stage_T(smem, rF, g.Aop, N * N, Kp, k0, bar);
+        else stage_T(smem, rF, g.F, 2 * Q, Kp, k0, bar);
+        stage_T(smem, rV, g.Vn, 3 * R, Kp, k0, bar);
+      }
       if (MODE != 0 && !LIN) stage_T(smem, rB, g.Bm, 4, Kp, k0, bar);
       stage_I<T>(smem, NT, 0, g.code, 1, Kp, k0, bar);
     }
@@ -980,12 +1024,29 @@ __device__ __forceinline__ void stage_op_tile(const Geo<T> g, const T *cin, cons
   for (int n = 0; n < 3; ++n) nb[n] = active ? g.nbr[(size_t)n * Kp + k] : -1;
   int vid[3] = {0, 0, 0};
   if (MODE != 0 && active) { vid[0] = g.V0T[k]; vid[1] = g.V0T[Kp + k]; vid[2] = g.V0T[2 * Kp + k]; }
+  int ax = 0;
+  T src[N];                                       // the source terms at this stage's time
+  if constexpr (FXP) {                            // neighbours across inflow edges only
+    if (active) ax = g.aopE[k];
+    if (g.rhsM) {
+#pragma unroll
+      for (int i = 0; i < N; ++i) src[i] = T(0);
+      for (int m = 0; m < g.nTerms && active; ++m) {
+        const T gm = T(sc.gco[m]);
+#pragma unroll
+        for (int i = 0; i < N; ++i) src[i] += gm * g.rhsM[((size_t)m * N + i) * Kp + k];
+      }
+    }
+#pragma unroll
+    for (int n = 0; n < 3; ++n)
+      if (!((ax >> (22 + n)) & 1)) nb[n] = -1;
+  }
   pdl_wait();
   if (MODE != 0) reset_next<T>(g, lo, k, nTiles < 0 ? -1 : tile, nTiles);
   if (!staged) return;
   if (t == 0) {                                   // state rows after it
     stage_T(smem, rC, cin, N, Kp, k0, bar);
-    if (MODE != 2) stage_T(smem, rC0, c0, N, Kp, k0, bar);
+    if (MODE != 2 && !first) stage_T(smem, rC0, c0, N, Kp, k0, bar);
   }
   // neighbour coefficients: outside the block from global memory now, inside from shared later
   A cn[3][N];
@@ -1000,6 +1061,7 @@ __device__ __forceinline__ void stage_op_tile(const Geo<T> g, const T *cin, cons
   bool bad = false;
   if (active && ok) {
     A c[N];
+    T cdot[N];
     Acc<A> rhs[N];
 #pragma unroll
     for (int i = 0; i < N; ++i) { c[i] = as_arith<A>(srow<T>(smem, rC + i)[t]); rhs[i] = Acc<A>(A(0)); }
@@ -1008,6 +1070,11 @@ __device__ __forceinline__ void stage_op_tile(const Geo<T> g, const T *cin, cons
       if (nb[n] >= k0 && nb[n] < k0 + eb)
 #pragma unroll
         for (int j = 0; j < N; ++j) cn[n][j] = as_arith<A>(srow<T>(smem, rC + j)[nb[n] - k0]);
+    bool summed = false;   // cdot is done in fixed point; else the FP64 rows come from global memory
+    if constexpr (FXP)
+      summed = fx::element_cdot<P>(fx_tab<P>(), (const Dig *)srow<T>(smem, rF) + t, (const Dig *)srow<T>(smem, rV) + t,
+                                   eb, ax, c, cn, irow<T>(smem, NT, 0)[t], cdot);
+    if (!summed) {
     if (RHS) {
       for (int m = 0; m < g.nTerms; ++m) {
         const A gm = A(sc.gco[m]);
@@ -1019,7 +1086,8 @@ __device__ __forceinline__ void stage_op_tile(const Geo<T> g, const T *cin, cons
 #pragma unroll
       for (int i = 0; i < N; ++i)
 #pragma unroll
-        for (int j = 0; j < N; ++j) rhs[i].fma(srow<T>(smem, rF + i * N + j)[t], c[j]);
+        for (int j = 0; j < N; ++j)
+          rhs[i].fma(FXP ? g.Aop[(size_t)(i * N + j) * Kp + k] : srow<T>(smem, rF + i * N + j)[t], c[j]);
     } else {
     // volume term (at p = 3, 12 points: unrolled by 3 to keep the body in the instruction cache)
 #pragma unroll(P >= 3 ? 3 : Q)
@@ -1044,7 +1112,7 @@ __device__ __forceinline__ void stage_op_tile(const Geo<T> g, const T *cin, cons
       const bool outOk = !EOP && ((code >> (6 + n)) & 1);
 #pragma unroll
       for (int r2 = 0; r2 < R; ++r2) {
-        const A v = as_arith<A>(srow<T>(smem, rV + n * R + r2)[t]);
+        const A v = as_arith<A>(FXP ? g.Vn[(size_t)(n * R + r2) * Kp + k] : srow<T>(smem, rV + n * R + r2)[t]);
         if (EOP && !(v < A(0) && nb[n] >= 0)) continue;
         Acc<A> tr(A(0));
         if (v > A(0) && outOk) {
@@ -1061,7 +1129,6 @@ __device__ __forceinline__ void stage_op_tile(const Geo<T> g, const T *cin, cons
       }
     }
     // mass solve
-    T cdot[N];
     if constexpr (sizeof(A) == 8 && !kFold) {
       A r[N];
 #pragma unroll
@@ -1077,6 +1144,11 @@ __device__ __forceinline__ void stage_op_tile(const Geo<T> g, const T *cin, cons
 #pragma unroll
       for (int i = 0; i < N; ++i) cdot[i] = T(rhs[i].get());
     }
+    }
+    if constexpr (FXP)
+      if (g.rhsM)
+#pragma unroll
+        for (int i = 0; i < N; ++i) cdot[i] += src[i];
     if (MODE == 2 && LIN) {
 #pragma unroll
       for (int i = 0; i < N; ++i) { out[(size_t)i * Kp + k] = cdot[i]; bad |= !finite_(cdot[i]); }
@@ -1094,7 +1166,8 @@ __device__ __forceinline__ void stage_op_tile(const Geo<T> g, const T *cin, cons
       T cnew[N];
 #pragma unroll
       for (int i = 0; i < N; ++i)
-        cnew[i] = w * srow<T>(smem, rC0 + i)[t] + (T(1) - w) * (srow<T>(smem, rC + i)[t] + tau * cdot[i]);
+        cnew[i] = first ? srow<T>(smem, rC + i)[t] + tau * cdot[i]
+                        : w * srow<T>(smem, rC0 + i)[t] + (T(1) - w) * (srow<T>(smem, rC + i)[t] + tau * cdot[i]);
       if (MODE == 0 || LIN) {
 #pragma unroll
         for (int i = 0; i < N; ++i) { out[(size_t)i * Kp + k] = cnew[i]; bad |= !finite_(cnew[i]); }
@@ -1573,6 +1646,9 @@ __device__ __forceinline__ void limit_dot_lin_tile(const Geo<T> g, const T *cin,
   constexpr int N = Dims<P>::N, NQ = 1;
   // staged rows: cDot, then N(N-1) rows of Q_k or the 4 rows of B, then c^n and c^(s-1)
   const bool fly = g.mtOnTheFly != 0;
+  const bool first = sc.omega == 0.0;   // c^n has no part in this stage: not read
+  // FP64 with stored rows and the global shift: the sums of products in fixed point
+  const bool fxOn = std::is_same_v<T, double> && !fly && li.shift && g.MTX != nullptr;
   const int NT = StageRows<T, P>::limdot_lin_rows(fly);
   extern __shared__ __align__(128) unsigned char smem[];
   uint64_t *bar = (uint64_t *)(smem + StageRows<T, P>::bar_offset(NT, 1, blockDim.x));
@@ -1586,21 +1662,23 @@ __device__ __forceinline__ void limit_dot_lin_tile(const Geo<T> g, const T *cin,
     if (t == 0) { mbar_init(bar, 1); mbar_fence_init(); }
     __syncthreads();
     if (t == 0) {
-      stage_expect<T>(bar, NT, 1);
+      stage_expect<T>(bar, NT - (first ? N : 0), 1);
       if (fly) stage_T(smem, rQ, g.Bm, 4, Kp, k0, bar);
-      else stage_T(smem, rQ, g.MT, N * (N - 1), Kp, k0, bar);
+      else stage_T(smem, rQ, fxOn ? (const T *)g.MTX : g.MT, N * (N - 1), Kp, k0, bar);
       stage_I<T>(smem, NT, 0, g.code, 1, Kp, k0, bar);
     }
   }
   const bool active = k < g.K;
   int vid[3] = {0, 0, 0};
   if (active) { vid[0] = g.V0T[k]; vid[1] = g.V0T[Kp + k]; vid[2] = g.V0T[2 * Kp + k]; }
+  int mx = -1;
+  if (fxOn && active) mx = g.mtE[k];
   pdl_wait();
   reset_next<T>(g, lo, k, nTiles < 0 ? -1 : tile, nTiles);
   if (!staged) return;
   if (t == 0) {
     stage_T(smem, rD, (const T *)tbuf, N, Kp, k0, bar);
-    stage_T(smem, rC0, c0, N, Kp, k0, bar);
+    if (!first) stage_T(smem, rC0, c0, N, Kp, k0, bar);
     stage_T(smem, rC, cin, N, Kp, k0, bar);
   }
   if (li.shift) load_shifts<T>(li.slots + slot_base(g, li.nc, tile), li.nc, sh);
@@ -1614,6 +1692,16 @@ __device__ __forceinline__ void limit_dot_lin_tile(const Geo<T> g, const T *cin,
     T cd[N], u[N], du[N];
 #pragma unroll
     for (int i = 0; i < N; ++i) cd[i] = srow<T>(smem, rD + i)[t];
+    bool limited = false;   // cd is done in fixed point
+    if constexpr (std::is_same_v<T, double>)
+      if (fxOn) {
+        T lo3[3], hi3[3];
+#pragma unroll
+        for (int n = 0; n < 3; ++n) { lo3[n] = vkey_inv<T>(kv.v[0][0][n]); hi3[n] = vkey_inv<T>(kv.v[0][1][n]); }
+        limited = fx::linear_cdot_limit<P>(fx_tab<P>(), lo3, hi3, sh[0], sh[1], (const Dig *)srow<T>(smem, rQ) + t,
+                                           kBlock, mx, cd);
+      }
+    if (!limited) {
     lin_u3<T, P>(cd, u);
     const int dmask = (irow<T>(smem, NT, 0)[t] >> 9) & 7;
     const T nan3[3] = {T(NAN), T(NAN), T(NAN)};
@@ -1650,16 +1738,21 @@ __device__ __forceinline__ void limit_dot_lin_tile(const Geo<T> g, const T *cin,
         for (int i = 0; i < N; ++i) {
           Acc<T> s(cd[i]);
 #pragma unroll
-          for (int j = 1; j < N; ++j) s.fma(srow<T>(smem, rQ + i * (N - 1) + (j - 1))[t], du[j]);
+          for (int j = 1; j < N; ++j) {
+            const int row = i * (N - 1) + (j - 1);
+            s.fma(fxOn ? g.MT[(size_t)row * Kp + k] : srow<T>(smem, rQ + row)[t], du[j]);
+          }
           cd[i] = s.get();
         }
       }
+    }
     }
     const T w = T(sc.omega), tau = T(sc.tau);
     T cnew[N];
 #pragma unroll
     for (int i = 0; i < N; ++i)
-      cnew[i] = w * srow<T>(smem, rC0 + i)[t] + (T(1) - w) * (srow<T>(smem, rC + i)[t] + tau * cd[i]);
+      cnew[i] = first ? srow<T>(smem, rC + i)[t] + tau * cd[i]
+                      : w * srow<T>(smem, rC0 + i)[t] + (T(1) - w) * (srow<T>(smem, rC + i)[t] + tau * cd[i]);
 #pragma unroll
     for (int i = 0; i < N; ++i) { out[(size_t)i * Kp + k] = cnew[i]; bad |= !finite_(cnew[i]); }
     q0 = lin_mean<T, P>(cnew);
@@ -1674,13 +1767,47 @@ k_limit_dot_lin(const Geo<T> g, const T *cin, const T *c0, const T *tbuf,
   limit_dot_lin_tile<T, P>(g, cin, c0, tbuf, out, li, lo, sc, blockIdx.x);
 }
 
+// One element's coefficients limited in place.
+template <typename T, int P>
+__device__ __forceinline__ void limit_lin_element(const LimIn<T> &li, const VKeys<T, 1> &kv, const T *sh, int dmask,
+                                                  const T data[3], T *c) {
+  constexpr int N = Dims<P>::N, NQ = 1;
+  const Tab<T, P> &tb = tab<T, P>();
+  T u[N], du[N];
+  bool limited = false;   // c is done in fixed point
+  if constexpr (std::is_same_v<T, double>)
+    if (li.shift) {
+      T lo3[3], hi3[3];
+#pragma unroll
+      for (int n = 0; n < 3; ++n) { lo3[n] = vkey_inv<T>(kv.v[0][0][n]); hi3[n] = vkey_inv<T>(kv.v[0][1][n]); }
+      limited = fx::linear_limit<P>(fx_tab<P>(), lo3, hi3, sh[0], sh[1], dmask, data, c);
+    }
+  if (!limited) {
+  lin_u3<T, P>(c, u);
+  if (lin_alpha<T, P, NQ>(li, kv, sh, u, dmask, data, du)) {
+    // limited: u - du is the linear Taylor polynomial (u_0, alpha u_1, alpha u_2); back in the
+    // modal basis that is the first three columns of DM^-1 (3N multiply-adds instead of the
+    // rows u_3.. and DM^-1 du, N(N-1) + 3(N-3))
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+      Acc<T> s(T(0));
+      s.fma(tb.DMinv[i][0], u[0]);
+      if constexpr (N > 1) {
+        s.fma(tb.DMinv[i][1], u[1] - du[1]);
+        s.fma(tb.DMinv[i][2], u[2] - du[2]);
+      }
+      c[i] = s.get();
+    }
+  }
+  }
+}
+
 // Solution limiter for the linear limiter (core/applySlopeLimiterDisc.m:77-86 without the
 // Taylor round trip): c <- c - DM^-1 du.
 template <typename T, int P>
 __device__ __forceinline__ void limit_lin_tile(const Geo<T> g, const T *cbuf, T *out, const LimIn<T> li,
             const StageScalars sc, const int tile) {
   constexpr int N = Dims<P>::N, NQ = 1;
-  const Tab<T, P> &tb = tab<T, P>();
   __shared__ T sh[2];
   const int t = threadIdx.x, k = tile * kBlock + t;
   pdl_trigger();
@@ -1708,23 +1835,7 @@ __device__ __forceinline__ void limit_lin_tile(const Geo<T> g, const T *cbuf, T 
   load_vkeys<T, NQ>(g, li, vid, kv);
   __syncthreads();
   if (!active) return;
-  T u[N], du[N];
-  lin_u3<T, P>(c, u);
-  if (lin_alpha<T, P, NQ>(li, kv, sh, u, dmask, data, du)) {
-    // limited: u - du is the linear Taylor polynomial (u_0, alpha u_1, alpha u_2); back in the
-    // modal basis that is the first three columns of DM^-1 (3N multiply-adds instead of the
-    // rows u_3.. and DM^-1 du, N(N-1) + 3(N-3))
-#pragma unroll
-    for (int i = 0; i < N; ++i) {
-      Acc<T> s(T(0));
-      s.fma(tb.DMinv[i][0], u[0]);
-      if constexpr (N > 1) {
-        s.fma(tb.DMinv[i][1], u[1] - du[1]);
-        s.fma(tb.DMinv[i][2], u[2] - du[2]);
-      }
-      c[i] = s.get();
-    }
-  }
+  limit_lin_element<T, P>(li, kv, sh, dmask, data, c);
   bool bad = false;
 #pragma unroll
   for (int i = 0; i < N; ++i) { out[(size_t)i * Kp + k] = c[i]; bad |= !finite_(c[i]); }

@@ -66,6 +66,11 @@ struct dgadv_handle {
   bool elemOp = true;
   void *Aop = nullptr;
   int aopVersion = -1;
+  // FP64: digits of Aop, Vn and the linear limiter's correction rows, with their exponents
+  // (dgadv_fixed.cuh)
+  void *AopX = nullptr, *VnX = nullptr, *MTX = nullptr;
+  int *aopE = nullptr, *mtE = nullptr;
+  void *rhsM = nullptr;                // FP64: the source terms with hatM^-1 applied
   // linked stepping (dgadv_link): this handle steps the handles in `linked` together with itself,
   // one launch per stage kernel; a handle in another's list has that handle as linkedTo
   std::vector<dgadv_handle *> linked;
@@ -219,6 +224,7 @@ struct PrecOps {
   // host FP64 -> stored reals (n values), written to dst (host memory of n * realBytes)
   void (*to_real)(const double *src, size_t n, void *dst);
   cudaError_t (*upload_tables)(int p, const RefTables &rt);   // constant tables of degree p
+  cudaError_t (*upload_tables_more)(int p, const RefTables &rt);   // ... of a second unit's copies (or null)
   cudaError_t (*set_smem)(int p);                             // opt-in shared memory sizes
   cudaError_t (*step)(dgadv_handle *h, double t0, double tau);
   cudaError_t (*step_fused)(dgadv_handle *h, double t0, double tau, bool firstOfCall);
@@ -283,6 +289,7 @@ void velocity_factors(const dgadv_handle *h, const double *u1, const double *u2,
                       std::vector<double> &F, std::vector<double> &Vn);
 
 const PrecOps &ops_fp64();
+PrecOps add_fp64_multi(PrecOps o);   // the persistent and linked steps (a unit of their own)
 const PrecOps &ops_fp32();
 const PrecOps &ops_df32_p01();   // df32 kernels compile per degree (three units in parallel)
 const PrecOps &ops_df32_p2();

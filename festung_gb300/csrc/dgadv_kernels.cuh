@@ -48,6 +48,24 @@ template <typename T, int P> struct Tab {
   T Fphi[3][R][N];
 };
 
+// One factor of a fixed-point sum (dgadv_fixed.cuh): h 2^29 + l.
+struct alignas(8) Dig {
+  int h, l;
+};
+// Tables of the FP64 stage kernels in digits, each entry scaled so that the sums it enters stay
+// below 1: thetaPhi by 2^-eT (the largest row sum over j), Fphi by 2^-eF (the largest sum over the
+// nine or so edge points), row i of DM by 2^-eDM[i] (its sum), row i of DMi, the first three
+// columns of DM^-1 with column j times 2^eDM[j], by 2^-eDMi[i].
+template <int P> struct FxTab {
+  static constexpr int N = Dims<P>::N, R = Dims<P>::R;
+  Dig thetaPhi[3][3][R][N];
+  Dig Fphi[3][R][N];
+  Dig DM[N][N];
+  Dig DMi[N][3];
+  int eT, eF;
+  int eDM[N < 3 ? 3 : N], eDMi[N];
+};
+
 // Static per-element data of one mesh (device pointers, SoA with stride Kp).
 template <typename T> struct Geo {
   int K, Kp, numV, Vp;
@@ -71,6 +89,11 @@ template <typename T> struct Geo {
   int nTerms;
   int timeFn[4];
   const int *instOf; // ensembles: instance of each block of kBlock elements (null: one instance)
+  // FP64 in fixed point (null: FP64 arithmetic): digits of Aop, Vn and the linear limiter's MT, and
+  // their exponents per element
+  const Dig *AopX, *VnX, *MTX;
+  const int *aopE, *mtE;
+  const T *rhsM;     // FP64: rhs with hatM^-1 applied, for the element operator (null without terms)
   const int *permv;  // Kp       caller's index of each element (ties of the limiter adjoint)
   int nInst;         // instances; each has its own global-extreme slots
 };

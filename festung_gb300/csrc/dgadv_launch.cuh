@@ -9,7 +9,66 @@
 
 namespace dgadv {
 
-template <typename T, int P>
+// A table entry x 2^-E as digits, to the nearest.
+static Dig host_digits(double x, int E) {
+  const long long X = std::llrint(std::ldexp(x, fx::kW - E));
+  Dig d;
+  d.l = (int)((uint32_t)X << 3) >> 3;
+  d.h = (int)((X - d.l) >> 29);
+  return d;
+}
+// The least E with x <= 2^E.
+static int host_exponent(double x) {
+  int e = 0;
+  if (x > 0.0 && std::frexp(x, &e) == 0.5) --e;
+  return e;
+}
+// The digit tables (FxTab) from the FP64 tables.
+template <int P>
+static cudaError_t upload_digits(const Tab<double, P> &t) {
+  constexpr int N = Dims<P>::N, R = Dims<P>::R;
+  FxTab<P> f;
+  double rowT = 0.0, sumF = 0.0;
+  for (int n = 0; n < 3; ++n)
+    for (int np = 0; np < 3; ++np)
+      for (int r = 0; r < R; ++r) {
+        double s = 0.0;
+        for (int j = 0; j < N; ++j) s += std::fabs(t.thetaPhi[n][np][r][j]);
+        rowT = std::max(rowT, s);
+      }
+  for (int i = 0; i < N; ++i) {
+    double s = 0.0;
+    for (int n = 0; n < 3; ++n)
+      for (int r = 0; r < R; ++r) s += std::fabs(t.Fphi[n][r][i]);
+    sumF = std::max(sumF, s);
+  }
+  f.eT = host_exponent(rowT);
+  f.eF = host_exponent(sumF);
+  for (int n = 0; n < 3; ++n)
+    for (int r = 0; r < R; ++r)
+      for (int i = 0; i < N; ++i) {
+        f.Fphi[n][r][i] = host_digits(t.Fphi[n][r][i], f.eF);
+        for (int np = 0; np < 3; ++np) f.thetaPhi[n][np][r][i] = host_digits(t.thetaPhi[n][np][r][i], f.eT);
+      }
+  for (int i = 0; i < (N < 3 ? 3 : N); ++i) {
+    double s = 0.0;
+    for (int j = 0; i < N && j < N; ++j) s += std::fabs(t.DM[i][j]);
+    f.eDM[i] = host_exponent(s);
+    for (int j = 0; i < N && j < N; ++j) f.DM[i][j] = host_digits(t.DM[i][j], f.eDM[i]);
+  }
+  for (int i = 0; i < N; ++i) {
+    double c[3], s = 0.0;
+    for (int j = 0; j < 3; ++j) {
+      c[j] = j < N ? std::ldexp(t.DMinv[i][j], f.eDM[j]) : 0.0;
+      s += std::fabs(c[j]);
+    }
+    f.eDMi[i] = host_exponent(s);
+    for (int j = 0; j < 3; ++j) f.DMi[i][j] = host_digits(c[j], f.eDMi[i]);
+  }
+  return cudaMemcpyToSymbol(fx_symbol<P>(), &f, sizeof(f));
+}
+
+template <typename T, int P, bool DIGITS = std::is_same_v<T, double>>
 static cudaError_t upload_tables(const RefTables &rt) {
   Tab<T, P> t;
   constexpr int N = Dims<P>::N, Q = Dims<P>::Q, R = Dims<P>::R;
@@ -74,14 +133,18 @@ static cudaError_t upload_tables(const RefTables &rt) {
   for (int n = 0; n < 3; ++n)
     for (int r = 0; r < R; ++r)
       for (int i = 0; i < N; ++i) t.Fphi[n][r][i] = T(lfold(&rt.phi1D[(n * R + r) * N], i));
+  if constexpr (DIGITS) {
+    const cudaError_t e = upload_digits<P>(t);
+    if (e != cudaSuccess) return e;
+  }
   return cudaMemcpyToSymbol(tab_symbol<T, P>(), &t, sizeof(t));
 }
 
 // The element operator (kOpElement) is in use: FP64 or double-float, enabled, built for the
-// current velocity and no source terms (with them the mass solve is not folded); a
+// current velocity; with source terms FP64 only, whose rows keep them with hatM^-1 applied; a
 // double-float handle with the FP32 operator keeps that one.
 static bool element_operator_on(const dgadv_handle *h) {
-  return h->Aop && h->elemOp && h->aopVersion == h->velVersion && !(h->nTerms > 0 && h->rhs) && !h->opFp32;
+  return h->Aop && h->elemOp && h->aopVersion == h->velVersion && (!(h->nTerms > 0 && h->rhs) || h->rhsM) && !h->opFp32;
 }
 template <typename T> constexpr bool kHasElementOperator = std::is_same_v<T, double> || std::is_same_v<T, df32>;
 
@@ -98,6 +161,9 @@ static Geo<T> make_geo(const dgadv_handle *h) {
   g.nInst = h->nInst;
   g.mtOnTheFly = h->mtOnTheFly ? 1 : 0;
   g.permv = h->perm;
+  g.AopX = (const Dig *)h->AopX; g.VnX = (const Dig *)h->VnX; g.MTX = (const Dig *)h->MTX;
+  g.aopE = h->aopE; g.mtE = h->mtE;
+  g.rhsM = h->nTerms > 0 ? (const T *)h->rhsM : nullptr;
   return g;
 }
 
@@ -280,14 +346,14 @@ template <typename T, int P, int MODE, bool RHS, bool LIN>
 static auto stage_kernel(const dgadv_handle *h) -> decltype(&k_stage_op<T, P, MODE, RHS, LIN, kOpPlain>) {
   if constexpr (std::is_same_v<T, df32>)
     if (h->opFp32) return &k_stage_op<T, P, MODE, RHS, LIN, kOpFp32>;
-  if constexpr (kHasElementOperator<T> && !RHS)
-    if (element_operator_on(h)) return &k_stage_op<T, P, MODE, RHS, LIN, kOpElement>;
+  if constexpr (kHasElementOperator<T> && (!RHS || std::is_same_v<T, double>))   // FP64 adds the terms itself
+    if (element_operator_on(h)) return &k_stage_op<T, P, MODE, false, LIN, kOpElement>;
   return &k_stage_op<T, P, MODE, RHS, LIN, kOpPlain>;
 }
 // Its staged rows.
 template <typename T, int P>
 static int stage_rows(const dgadv_handle *h, int mode, bool lin, bool rhs) {
-  return StageRows<T, P>::op(mode, lin, kHasElementOperator<T> && !rhs && element_operator_on(h));
+  return StageRows<T, P>::op(mode, lin, kHasElementOperator<T> && (!rhs || std::is_same_v<T, double>) && element_operator_on(h));
 }
 
 template <typename T, int P>
@@ -580,9 +646,32 @@ static cudaError_t dispatch_build_element_operator(dgadv_handle *h) {
       case 2: if constexpr ((MASK & 4) != 0) k_build_element_operator<T, 2><<<grid, kBlock, 0, h->stream>>>(g, (T *)h->Aop); break;
       case 3: if constexpr ((MASK & 8) != 0) k_build_element_operator<T, 3><<<grid, kBlock, 0, h->stream>>>(g, (T *)h->Aop); break;
     }
+    if constexpr (std::is_same_v<T, double>) {
+      auto fix = [&](auto P_) {
+        constexpr int P = decltype(P_)::value;
+        k_fix_operator<P><<<grid, kBlock, 0, h->stream>>>(h->K, h->Kp, (const double *)h->Aop, (const double *)h->Vn,
+                                                          h->nbr, (Dig *)h->AopX, (Dig *)h->VnX, h->aopE);
+      };
+      switch (h->p) {
+        case 0: fix(std::integral_constant<int, 0>()); break;
+        case 1: fix(std::integral_constant<int, 1>()); break;
+        case 2: fix(std::integral_constant<int, 2>()); break;
+        case 3: fix(std::integral_constant<int, 3>()); break;
+      }
+    }
     return cudaGetLastError();
   }
   return cudaErrorNotSupported;
+}
+
+// The digits of the linear limiter's correction rows (FP64, p >= 2).
+template <typename T>
+static cudaError_t dispatch_fix_correction(dgadv_handle *h) {
+  static_assert(std::is_same_v<T, double>, "");
+  const int grid = (h->K + kBlock - 1) / kBlock;
+  if (h->p == 2) k_fix_correction<2><<<grid, kBlock, 0, h->stream>>>(h->K, h->Kp, (const double *)h->MT, (Dig *)h->MTX, h->mtE);
+  else if (h->p == 3) k_fix_correction<3><<<grid, kBlock, 0, h->stream>>>(h->K, h->Kp, (const double *)h->MT, (Dig *)h->MTX, h->mtE);
+  return cudaGetLastError();
 }
 
 template <typename T, int MASK, bool FUSED>
@@ -594,6 +683,7 @@ static PrecOps make_ops() {
   o.fused = FUSED;
   o.to_real = to_real<T>;
   o.upload_tables = upload_tables_p<T, MASK>;
+  o.upload_tables_more = nullptr;
   o.set_smem = set_smem_p<T, MASK, FUSED>;
   o.step = dispatch_step<T, MASK>;
   o.step_fused = dispatch_step_fused<T, MASK, FUSED>;

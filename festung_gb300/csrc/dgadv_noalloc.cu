@@ -160,8 +160,8 @@ extern "C" int dgadv_limit_linear_noalloc(int32_t p, int32_t numT, int32_t numV,
       RefTables rt;
       std::string err;
       if (!build_ref_tables(p, rt, err)) return DGADV_EINVAL;
-      const cudaError_t e = p == 1 ? upload_tables<double, 1>(rt)
-                          : p == 2 ? upload_tables<double, 2>(rt) : upload_tables<double, 3>(rt);
+      const cudaError_t e = p == 1 ? upload_tables<double, 1, false>(rt)
+                          : p == 2 ? upload_tables<double, 2, false>(rt) : upload_tables<double, 3, false>(rt);
       if (e != cudaSuccess) return DGADV_ECUDA;
       g_noalloc_tables[dev][p] = true;
     }

@@ -327,12 +327,21 @@ static int create_impl(const dgadv_mesh *mesh, const dgadv_params *prm, const st
     if (h->device < 0 || h->device >= 64) { h->err = "device ordinal out of range"; return DGADV_EINVAL; }
     if (!implicit && !g_tab_loaded[h->device][pi][h->p]) {   // implicit handles use their own tables
       cudaError_t e = ops(h).upload_tables(h->p, h->tables);
+      if (e == cudaSuccess && ops(h).upload_tables_more) e = ops(h).upload_tables_more(h->p, h->tables);
       if (e != cudaSuccess) { h->err = std::string("table upload: ") + cudaGetErrorString(e); return DGADV_ECUDA; }
       e = ops(h).set_smem(h->p);
       if (e == cudaSuccess && ops(h).persist_attributes) e = ops(h).persist_attributes(h->p);
       if (e != cudaSuccess) { h->err = std::string("kernel attributes: ") + cudaGetErrorString(e); return DGADV_ECUDA; }
       g_tab_loaded[h->device][pi][h->p] = true;
     }
+  }
+  if (ops(h).fix_correction && h->limdot && h->limType == DGADV_LIM_LINEAR) {
+    const size_t nQ = (size_t)N * (N - 1) * Kp * 8;
+    if ((st = dev_alloc(h, &h->MTX, nQ))) return st;
+    if ((st = dev_alloc(h, (void **)&h->mtE, (size_t)Kp * 4))) return st;
+    DG_CUDA(cudaMemset(h->MTX, 0, nQ));
+    DG_CUDA(cudaMemset(h->mtE, 0, (size_t)Kp * 4));
+    DG_CUDA(ops(h).fix_correction(h));
   }
   DG_CUDA(cudaDeviceSynchronize());
   return DGADV_OK;
@@ -466,6 +475,19 @@ extern "C" int dgadv_set_source_terms(dgadv_handle *h, int32_t nTerms, const int
   if (!h->rhs && (st = dev_alloc(h, &h->rhs, 4 * (size_t)N * Kp * w))) return st;
   if (cDV0T && !h->cDV0T && (st = dev_alloc(h, &h->cDV0T, 4 * (size_t)3 * Kp * w))) return st;
   if ((st = upload_real(h, h->rhs, r))) return st;
+  if (h->prec == DGADV_FP64 && !(h->flags & DGADV_FLAG_IMPLICIT)) {   // with hatM^-1 applied
+    if (!h->rhsM && (st = dev_alloc(h, &h->rhsM, 4 * (size_t)N * Kp * w))) return st;
+    std::vector<double> rm(r.size(), 0.0);
+    for (int m = 0; m < nTerms; ++m)
+      for (int i = 0; i < N; ++i)
+        for (int j = 0; j < N; ++j) {
+          const double a = h->tables.hatMinv[i * N + j];
+          const double *src = &r[((size_t)m * N + j) * Kp];
+          double *dst = &rm[((size_t)m * N + i) * Kp];
+          for (int k = 0; k < K; ++k) dst[k] += a * src[k];
+        }
+    if ((st = upload_real(h, h->rhsM, rm))) return st;
+  }
   if (cDV0T && (st = upload_real(h, h->cDV0T, d))) return st;
   if (!cDV0T && h->cDV0T) DG_CUDA(cudaMemset(h->cDV0T, 0, 4 * (size_t)3 * Kp * w));
   return DGADV_OK;
@@ -710,6 +732,15 @@ int dgadv::refresh_element_operator(dgadv_handle *h) {
     int st;
     if ((st = dev_alloc(h, &h->Aop, (size_t)h->N * h->N * h->Kp * o.realBytes))) return st;
     DG_CUDA(cudaMemset(h->Aop, 0, (size_t)h->N * h->N * h->Kp * o.realBytes));
+    if (h->prec == DGADV_FP64) {   // its digits (padding elements: zero)
+      const size_t nA = (size_t)h->N * h->N * h->Kp * 8, nV = (size_t)3 * h->R * h->Kp * 8, nE = (size_t)h->Kp * 4;
+      if ((st = dev_alloc(h, &h->AopX, nA))) return st;
+      if ((st = dev_alloc(h, &h->VnX, nV))) return st;
+      if ((st = dev_alloc(h, (void **)&h->aopE, nE))) return st;
+      DG_CUDA(cudaMemset(h->AopX, 0, nA));
+      DG_CUDA(cudaMemset(h->VnX, 0, nV));
+      DG_CUDA(cudaMemset(h->aopE, 0, nE));
+    }
   }
   DG_CUDA(o.build_element_operator(h));
   // captured steps keep their kernels: they are recaptured once the operator comes into use
