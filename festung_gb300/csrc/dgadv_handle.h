@@ -267,6 +267,8 @@ inline bool use_persistent(const dgadv_handle *h) {
   return (h->flags & DGADV_FLAG_PERSIST) && !(h->flags & DGADV_FLAG_FUSE) && h->p >= 1 &&
          (!h->lim || h->limType == DGADV_LIM_LINEAR) && h->nTerms == 0;
 }
+  // FP64: the digits of the linear limiter's correction rows (null: not used)
+  cudaError_t (*fix_correction)(dgadv_handle *h);
 
 const PrecOps &ops_of(const dgadv_handle *h);
 

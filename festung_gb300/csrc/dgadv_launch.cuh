@@ -708,3 +708,5 @@ static PrecOps make_ops() {
 }
 
 }  // namespace dgadv
+  o.fix_correction = nullptr;
+  if constexpr (std::is_same_v<T, double>) o.fix_correction = dispatch_fix_correction<T>;
