@@ -250,6 +250,8 @@ struct PrecOps {
   cudaError_t (*from_f64)(dgadv_handle *h, void *dst, const double *src, size_t n);
   // the element operator of every element from the velocity factors (null: not built)
   cudaError_t (*build_element_operator)(dgadv_handle *h);
+  // FP64: the digits of the linear limiter's correction rows (null: not used)
+  cudaError_t (*fix_correction)(dgadv_handle *h);
   // transport problem (null: not built for this type)
   cudaError_t (*tr_stage)(dgadv_handle *h, const TrStageArgs &a);
   cudaError_t (*tr_convert)(dgadv_handle *h, const void *in, void *out, const void *hQ, int toConc);
@@ -267,8 +269,6 @@ inline bool use_persistent(const dgadv_handle *h) {
   return (h->flags & DGADV_FLAG_PERSIST) && !(h->flags & DGADV_FLAG_FUSE) && h->p >= 1 &&
          (!h->lim || h->limType == DGADV_LIM_LINEAR) && h->nTerms == 0;
 }
-  // FP64: the digits of the linear limiter's correction rows (null: not used)
-  cudaError_t (*fix_correction)(dgadv_handle *h);
 
 const PrecOps &ops_of(const dgadv_handle *h);
 

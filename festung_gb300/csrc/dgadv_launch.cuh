@@ -701,6 +701,8 @@ static PrecOps make_ops() {
   o.copy = copy_state;
   o.from_f64 = from_f64<T>;
   o.build_element_operator = kHasElementOperator<T> ? dispatch_build_element_operator<T, MASK> : nullptr;
+  o.fix_correction = nullptr;
+  if constexpr (std::is_same_v<T, double>) o.fix_correction = dispatch_fix_correction<T>;
   o.tr_stage = nullptr;
   o.tr_convert = nullptr;
   o.tr_mask = nullptr;
@@ -708,5 +710,3 @@ static PrecOps make_ops() {
 }
 
 }  // namespace dgadv
-  o.fix_correction = nullptr;
-  if constexpr (std::is_same_v<T, double>) o.fix_correction = dispatch_fix_correction<T>;
