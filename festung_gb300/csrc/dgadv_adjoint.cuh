@@ -62,7 +62,6 @@ k_adj_stage(const Geo<T> g, const T *muIn, const T *mpIn, const T *cs, T *__rest
   constexpr int N = Dims<P>::N, Q = Dims<P>::Q, R = Dims<P>::R;
   const Tab<T, P> &tb = tab<T, P>();
   const int k = blockIdx.x * kBlock + threadIdx.x;
-  pdl_trigger();
   if (k >= g.K) return;
   const int Kp = g.Kp;
   const T w = T(a.omega), coef = T((1.0 - a.omega) * a.tau);
@@ -84,6 +83,7 @@ k_adj_stage(const Geo<T> g, const T *muIn, const T *mpIn, const T *cs, T *__rest
 #pragma unroll
     for (int r = 0; r < R; ++r) V2[n][r] = nb[n] >= 0 ? g.Vn[(size_t)(nk[n] * R + r) * Kp + nb[n]] : T(0);
   pdl_wait();
+  pdl_trigger();
   // every load of the stage's data up front: the kernel is latency-bound otherwise
   T mu[N], c[N], cn[3][N], mu2[3][N];
   SensAcc<T> sF[2 * Q], sV[3 * R];
@@ -220,6 +220,7 @@ __device__ __forceinline__ void adj_edge_role(const Geo<T> &g, const AdjSplitIn<
     V2[r] = nb >= 0 ? g.Vn[(size_t)(nk * R + r) * Kp + nb] : T(0);
   }
   pdl_wait();
+  pdl_trigger();
   T c[N], mp[N], cn[N], mu2[N];
   SensAcc<T> sV[R];
 #pragma unroll
@@ -286,6 +287,7 @@ __device__ __forceinline__ void adj_volume_role(const Geo<T> &g, const AdjSplitI
 #pragma unroll
   for (int i = 0; i < 2 * Q; ++i) F[i] = g.F[(size_t)i * Kp + e];
   pdl_wait();
+  pdl_trigger();
   T c[N], mp[N];
   SensAcc<T> sF[2 * Q];
 #pragma unroll
@@ -328,7 +330,6 @@ k_adj_stage_split(const Geo<T> g, const T *muIn, const T *mpIn, const T *cs, T *
   constexpr int N = Dims<P>::N;
   constexpr int NL = (N + 3) / 4;   // coefficients each role stores, at most
   __shared__ T part[4][N][32 * W];
-  pdl_trigger();
   const int warp = threadIdx.x / 32, role = warp / W;
   const int lane = (warp % W) * 32 + threadIdx.x % 32;   // element of the CTA
   const int k = blockIdx.x * (32 * W) + lane;
@@ -414,7 +415,6 @@ k_lim_vjp(const Geo<T> g, const T *x, const T *lamIn, T *__restrict__ lamOut, co
   const Tab<T, P> &tb = tab<T, P>();
   __shared__ T sh[2];
   const int k = blockIdx.x * kBlock + threadIdx.x;
-  pdl_trigger();
   const bool active = k < g.K;
   const int Kp = g.Kp;
   int vid[3] = {0, 0, 0}, pos[3] = {0, 0, 0}, dmask = 0;
@@ -448,6 +448,7 @@ k_lim_vjp(const Geo<T> g, const T *x, const T *lamIn, T *__restrict__ lamOut, co
     for (int i = 0; i < N * (N - 1); ++i) mtv[i] = active ? g.MT[(size_t)i * Kp + k] : T(0);
   }
   pdl_wait();
+  pdl_trigger();
   // blocks past the last element tile (SNEXT grids cover the vertices) use the last tile's
   // instance for the global extremes
   const int tile = min((int)blockIdx.x, (g.K - 1) / kBlock);
@@ -618,7 +619,6 @@ k_lim_choice(const Geo<T> g, const T *x, const LimIn<T> li, const StageScalars s
   constexpr int N = Dims<P>::N;
   __shared__ T sh[2];
   const int k = blockIdx.x * kBlock + threadIdx.x;
-  pdl_trigger();
   const bool active = k < g.K;
   const int Kp = g.Kp;
   int vid[3] = {0, 0, 0}, dmask = 0;
@@ -642,6 +642,7 @@ k_lim_choice(const Geo<T> g, const T *x, const LimIn<T> li, const StageScalars s
     }
   }
   pdl_wait();
+  pdl_trigger();
   const int tile = min((int)blockIdx.x, (g.K - 1) / kBlock);
   if (li.shift) load_shifts<T>(li.slots + slot_base(g, li.nc, tile), li.nc, sh);
   T xv[N];
@@ -718,7 +719,6 @@ k_lim_apply(const Geo<T> g, const T *x, const T *lamIn, T *__restrict__ lamOut, 
   constexpr int N = Dims<P>::N;
   const Tab<T, P> &tb = tab<T, P>();
   const int k = blockIdx.x * kBlock + threadIdx.x;
-  pdl_trigger();
   if (k >= g.K) return;
   const int Kp = g.Kp;
   const int pos[3] = {csrPos[k], csrPos[Kp + k], csrPos[2 * Kp + k]};
@@ -738,6 +738,7 @@ k_lim_apply(const Geo<T> g, const T *x, const T *lamIn, T *__restrict__ lamOut, 
     for (int i = 0; i < N * (N - 1); ++i) mtv[i] = g.MT[(size_t)i * Kp + k];
   }
   pdl_wait();
+  pdl_trigger();
   const int info = rec.info[k];
   const int ns = info & 3;
   T lam[N];
@@ -824,7 +825,6 @@ k_lim_vjp_gather(const Geo<T> g, T *lam, const int *slotT, const T *slotW) {
   constexpr int N = Dims<P>::N;
   const Tab<T, P> &tb = tab<T, P>();
   const int k = blockIdx.x * kBlock + threadIdx.x;
-  pdl_trigger();
   if (k >= g.K) return;
   const int Kp = g.Kp;
   const int vid[3] = {g.V0T[k], g.V0T[Kp + k], g.V0T[2 * Kp + k]};
@@ -835,6 +835,7 @@ k_lim_vjp_gather(const Geo<T> g, T *lam, const int *slotT, const T *slotW) {
     i1[n] = g.vptr[vid[n] + 1];
   }
   pdl_wait();
+  pdl_trigger();
   T acc = T(0);
   bool any = false;
 #pragma unroll
@@ -1055,12 +1056,12 @@ __global__ void __launch_bounds__(kBlock)
 k_vjp_scatter_hier(const Geo<T> g, const T *x, const LimOut<T> lo, T *__restrict__ qOut) {
   constexpr int N = Dims<P>::N, NQ = NCQ<P>::value;
   const int k = blockIdx.x * kBlock + threadIdx.x;
-  pdl_trigger();
   const bool active = k < g.K;
   const int Kp = g.Kp;
   int vid[3] = {0, 0, 0};
   if (active) { vid[0] = g.V0T[k]; vid[1] = g.V0T[Kp + k]; vid[2] = g.V0T[2 * Kp + k]; }
   pdl_wait();
+  pdl_trigger();
   reset_next<T>(g, lo, k);
   T qv[NQ];
 #pragma unroll
@@ -1143,7 +1144,6 @@ k_lim_vjp_hier(const Geo<T> g, const T *x, const T *lamIn, T *__restrict__ lamOu
   constexpr int N = Dims<P>::N, NQ = NCQ<P>::value;
   __shared__ T sh[2 * NQ];
   const int k = blockIdx.x * kBlock + threadIdx.x;
-  pdl_trigger();
   const bool active = k < g.K;
   const int Kp = g.Kp;
   int vid[3] = {0, 0, 0}, pos[3] = {-1, -1, -1}, dmask = 0;
@@ -1168,6 +1168,7 @@ k_lim_vjp_hier(const Geo<T> g, const T *x, const T *lamIn, T *__restrict__ lamOu
       for (int n = 0; n < 3; ++n) data[n] += gm * g.cDV0T[((size_t)m * 3 + n) * Kp + k];
     }
   pdl_wait();
+  pdl_trigger();
   if (li.shift) load_shifts<T>(li.slots + slot_base(g, li.nc), li.nc, sh);
   T xv[N], lraw[N];
 #pragma unroll
@@ -1378,7 +1379,6 @@ k_lim_vjp_strict(const Geo<T> g, const T *x, const T *lamIn, T *__restrict__ lam
   constexpr int N = Dims<P>::N, NQ = NCQ<P>::value;
   __shared__ T sh[2 * NQ];
   const int k = blockIdx.x * kBlock + threadIdx.x;
-  pdl_trigger();
   const bool active = k < g.K;
   const int Kp = g.Kp;
   int vid[3] = {0, 0, 0}, pos[3] = {-1, -1, -1}, dmask = 0;
@@ -1403,6 +1403,7 @@ k_lim_vjp_strict(const Geo<T> g, const T *x, const T *lamIn, T *__restrict__ lam
       for (int n = 0; n < 3; ++n) data[n] += gm * g.cDV0T[((size_t)m * 3 + n) * Kp + k];
     }
   pdl_wait();
+  pdl_trigger();
   if (li.shift) load_shifts<T>(li.slots + slot_base(g, li.nc), li.nc, sh);
   T xv[N], lraw[N];
 #pragma unroll
@@ -1583,7 +1584,6 @@ __global__ void __launch_bounds__(kBlock)
 k_lim_vjp_hier_gather(const Geo<T> g, T *lam, int nnz, const int *slotT, const T *slotW) {
   constexpr int N = Dims<P>::N;
   const int k = blockIdx.x * kBlock + threadIdx.x;
-  pdl_trigger();
   if (k >= g.K) return;
   const int Kp = g.Kp;
   const int vid[3] = {g.V0T[k], g.V0T[Kp + k], g.V0T[2 * Kp + k]};
@@ -1594,6 +1594,7 @@ k_lim_vjp_hier_gather(const Geo<T> g, T *lam, int nnz, const int *slotT, const T
 #pragma unroll
   for (int r = 0; r < 4; ++r) B[r] = g.Bm[(size_t)r * Kp + k];
   pdl_wait();
+  pdl_trigger();
   T acc[N];
   if (!hier_records<T, P>(k, i0, i1, nnz, slotT, slotW, acc)) return;
   const Affine<T> af = affine_from<T>(B[0], B[1], B[2], B[3]);

@@ -429,12 +429,67 @@ __device__ __forceinline__ bool nan_(double x) {
 }
 __device__ __forceinline__ bool nan_(const df32 &x) { return x.hi != x.hi || x.lo != x.lo; }
 
+// Whether a block of the stage operator works with its vertex table (blocks of kBlock elements), and
+// the block's empty key table at vtOff (a block barrier has to follow before scatter_quantities).
+// 32-bit keys only: a 64-bit minimum in shared memory is a compare-and-swap loop (measured: FP64
+// operator on 2048 triangles 7.2 -> 9.0 us).
+template <typename T> __device__ __forceinline__ bool vt_on() {
+  return sizeof(typename KeyOf<T>::type) == 4 && blockDim.x == kBlock;
+}
+// The block's vertex list: its bounds and this thread's vertex, read before the dependency wait.
+struct VtList {
+  int v0, nv, v;
+};
+template <typename T> __device__ __forceinline__ VtList vt_list(const Geo<T> &g, int tile) {
+  VtList l;
+  l.v0 = g.vtPtr[tile];
+  l.nv = g.vtPtr[tile + 1] - l.v0;
+  l.v = (int)threadIdx.x < l.nv ? g.vtIdx[l.v0 + threadIdx.x] : 0;
+  return l;
+}
+template <typename T>
+__device__ __forceinline__ void vt_reset(const Geo<T> &g, int nc, int vtOff) {
+  extern __shared__ __align__(128) unsigned char smem[];
+  auto *tk = (typename KeyOf<T>::type *)(smem + vtOff);
+  for (int s = 0; s < nc; ++s)
+    for (int i = threadIdx.x; i < g.vtMax; i += blockDim.x) {
+      tk[(2 * s) * g.vtMax + i] = vkey_max<T>();
+      tk[(2 * s + 1) * g.vtMax + i] = 0;
+    }
+}
+// The element's vertices: positions in its block's table, or ids.
+template <typename T>
+__device__ __forceinline__ void load_vertices(const Geo<T> &g, int k, bool local, int vid[3]) {
+#pragma unroll
+  for (int n = 0; n < 3; ++n) vid[n] = local ? (int)g.vtLoc[(size_t)n * g.Kp + k] : g.V0T[(size_t)n * g.Kp + k];
+}
+
 // Scatter of the element's centroid quantities to its vertices and the block's global extremes.
+//
+// With vtOff >= 0 (bytes into the dynamic shared memory) the keys are first gathered in the block's
+// vertex table there (vt_reset has cleared it, with a block barrier since), vid being positions in
+// the block's list; each vertex of the block then takes one atomic per key instead of one per
+// element around it: 128 elements touch about 80 vertices, so 1.3 atomics per element and key pair
+// instead of 6, on consecutive addresses.
 template <typename T, int NQ>
 __device__ __forceinline__ void scatter_quantities(const Geo<T> &g, const LimOut<T> &lo, const T *qv,
-                                                   const int vid[3], bool active, int tile = -1) {
+                                                   const int vid[3], bool active, int tile = -1, int vtOff = -1,
+                                                   const VtList vl = VtList{0, 0, 0}) {
   if (tile < 0) tile = blockIdx.x;
-  if (active) {
+  extern __shared__ __align__(128) unsigned char smem[];
+  if (active && vtOff >= 0) {
+    auto *tk = (typename KeyOf<T>::type *)(smem + vtOff);
+#pragma unroll
+    for (int s = 0; s < NQ; ++s) {
+      if (s >= lo.nc) break;
+      const auto key = vkey(qv[s]);
+#pragma unroll
+      for (int n = 0; n < 3; ++n) {
+        atomicMin(&tk[(2 * s) * g.vtMax + vid[n]], key);
+        atomicMax(&tk[(2 * s + 1) * g.vtMax + vid[n]], key);
+      }
+    }
+  } else if (active) {
 #pragma unroll
     for (int s = 0; s < NQ; ++s) {
       if (s >= lo.nc) break;
@@ -461,6 +516,18 @@ __device__ __forceinline__ void scatter_quantities(const Geo<T> &g, const LimOut
     if (lane == 0) { red[warp][2 * s] = mn; red[warp][2 * s + 1] = mx; }
   }
   __syncthreads();
+  if (vtOff >= 0) {
+    const auto *tk = (const typename KeyOf<T>::type *)(smem + vtOff);
+    for (int i = threadIdx.x; i < vl.nv; i += blockDim.x) {
+      const int v = i < (int)blockDim.x ? vl.v : g.vtIdx[vl.v0 + i];
+#pragma unroll
+      for (int s = 0; s < NQ; ++s) {
+        if (s >= lo.nc) break;
+        atomicMin(&lo.vkeys[(size_t)(2 * s) * g.Vp + v], tk[(2 * s) * g.vtMax + i]);
+        atomicMax(&lo.vkeys[(size_t)(2 * s + 1) * g.Vp + v], tk[(2 * s + 1) * g.vtMax + i]);
+      }
+    }
+  }
   if (threadIdx.x < lo.nc) {
     const int s = threadIdx.x;
     K_ mn = red[0][2 * s], mx = red[0][2 * s + 1];
@@ -636,9 +703,14 @@ __device__ __forceinline__ void stage_expect(uint64_t *bar, int nT, int nI) {
   mbar_expect_tx(bar, nT * blockDim.x * (uint32_t)sizeof(T) + nI * blockDim.x * (uint32_t)sizeof(int));
 }
 
-// Programmatic dependent launch: the next kernel in the stream may start its prologue (static
-// data only) once every block of this one has started; pdl_wait() blocks until the previous
-// kernel has completed and its writes are visible.
+// Programmatic dependent launch: pdl_wait() blocks until the previous kernel has completed and its
+// writes are visible; from pdl_trigger() on (in every block) the next kernel in the stream may start
+// its prologue (static data only).  Every kernel triggers right after its own wait, so that one
+// kernel at most waits beside the running one.  Triggered before the wait, a whole chain of small
+// kernels piles up on the SMs, each placed where the ones before it left room: their blocks end up
+// on few SMs, and a chain can run slower than without the early launch (four species on 8192
+// triangles, p = 1, FP64: 123 us per step so, 43 us now; 6498 triangles, p = 2, FP64: 45 and 23.5 us
+// per stage, 30 without dependent launch).
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 // A kernel in such a chain must not declare a buffer that earlier kernels of the chain write as
@@ -655,8 +727,8 @@ namespace dgadv {
 // dependency wait covers the kernel launched before it, not a copy-engine transfer queued in
 // between, so a cudaMemcpyAsync there is not ordered against the kernel that follows.
 static __global__ void k_copy16(const uint4 *src, uint4 *__restrict__ dst, size_t n) {
-  pdl_trigger();
   pdl_wait();
+  pdl_trigger();
   for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x)
     dst[i] = src[i];
 }
@@ -727,6 +799,71 @@ __device__ __forceinline__ void patch_minmax(const LimIn<T> &li, const VKeys<T, 
   }
 }
 
+// The same extremes from the block's table of shifted vertex extremes (load_patch).
+template <typename T> struct PatchView {
+  const T *pv;      // quantity s: minima at 2 s stride, maxima at (2 s + 1) stride
+  int stride;
+  int l[3];         // the element's positions in the table
+};
+template <typename T, int NQ>
+__device__ __forceinline__ void patch_minmax(const LimIn<T> &, const PatchView<T> &kv, const T *, int s,
+                                             const T valD[3], T mn[3], T mx[3]) {
+#pragma unroll
+  for (int n = 0; n < 3; ++n) {
+    mn[n] = fmin(kv.pv[(2 * s) * kv.stride + kv.l[n]], valD[n]);
+    mx[n] = fmax(kv.pv[(2 * s + 1) * kv.stride + kv.l[n]], valD[n]);
+  }
+}
+// The extremes alone (no boundary data).
+template <typename T>
+__device__ __forceinline__ void patch_extremes(const LimIn<T> &li, const VKeys<T, 1> &kv, const T *sh, T mn[3], T mx[3]) {
+  const T none[3] = {T(NAN), T(NAN), T(NAN)};
+  patch_minmax<T, 1>(li, kv, sh, 0, none, mn, mx);
+}
+template <typename T>
+__device__ __forceinline__ void patch_extremes(const LimIn<T> &, const PatchView<T> &kv, const T *, T mn[3], T mx[3]) {
+#pragma unroll
+  for (int n = 0; n < 3; ++n) { mn[n] = kv.pv[kv.l[n]]; mx[n] = kv.pv[kv.stride + kv.l[n]]; }
+}
+
+// The block's table of patch extremes at vtOff: each vertex's keys read, decoded and shifted
+// once per block (the elements around it would do so six times), by the thread that owns the
+// vertex.  Contains the global extremes' reduction (load_shifts) and two block barriers.
+template <typename T, int NQ>
+__device__ __forceinline__ void load_patch(const Geo<T> &g, const LimIn<T> &li, int tile, const VtList &vl, T *sh,
+                                           int vtOff) {
+  extern __shared__ __align__(128) unsigned char smem[];
+  T *pv = (T *)(smem + vtOff);
+  typename KeyOf<T>::type raw[NQ][2];
+  const int i0 = threadIdx.x;
+  if (i0 < vl.nv) {
+#pragma unroll
+    for (int s = 0; s < NQ; ++s)
+#pragma unroll
+      for (int m = 0; m < 2; ++m) raw[s][m] = s < li.nc ? li.vkeys[(size_t)(2 * s + m) * g.Vp + vl.v] : 0;
+  }
+  if (li.shift) load_shifts<T>(li.slots + slot_base(g, li.nc, tile), li.nc, sh);
+  __syncthreads();
+  for (int i = i0; i < vl.nv; i += blockDim.x) {
+    if (i != i0) {
+      const int v = g.vtIdx[vl.v0 + i];
+#pragma unroll
+      for (int s = 0; s < NQ; ++s)
+#pragma unroll
+        for (int m = 0; m < 2; ++m) raw[s][m] = s < li.nc ? li.vkeys[(size_t)(2 * s + m) * g.Vp + v] : 0;
+    }
+#pragma unroll
+    for (int s = 0; s < NQ; ++s) {
+      if (s >= li.nc) break;
+      T a = vkey_inv<T>(raw[s][0]), c = vkey_inv<T>(raw[s][1]);
+      if (li.shift) { a = (a - sh[2 * s + 1]) + sh[2 * s + 1]; c = (c + sh[2 * s]) - sh[2 * s]; }
+      pv[(2 * s) * g.vtMax + i] = a;
+      pv[(2 * s + 1) * g.vtMax + i] = c;
+    }
+  }
+  __syncthreads();
+}
+
 // Limit Taylor coefficients in place (linear / hierarchical vertex).  dataV0T: boundary values
 // at the three vertices for Dirichlet vertices (NaN means "no data").
 // Taylor basis functions of core/phiTaylorPhy.m at the element's vertices, phi[n][j] for the
@@ -768,8 +905,8 @@ __device__ __forceinline__ void taylor_vertex_basis(const Affine<T> &af, T phi[3
 
 // LT: the limiter type (0 linear, 1 hierarchical vertex, 2 strict), fixed per kernel so that
 // each kernel carries the code of one limiter only.
-template <typename T, int P, int NQ, int LT>
-__device__ __forceinline__ void limit_taylor(const LimIn<T> &li, const VKeys<T, NQ> &kv, const T *sh,
+template <typename T, int P, int NQ, int LT, typename KV>
+__device__ __forceinline__ void limit_taylor(const LimIn<T> &li, const KV &kv, const T *sh,
                                              const Affine<T> &af, int dmask, const T dataV0T[3], T *cT) {
   constexpr int N = Dims<P>::N;
   const T nan_ = T(NAN);
@@ -912,8 +1049,8 @@ template <typename T, int P> __device__ __forceinline__ T lin_mean(const T *c) {
   return s.get();
 }
 // alpha of the linear limiter from u, and the removed part du (returns false if alpha == 1).
-template <typename T, int P, int NQ>
-__device__ __forceinline__ bool lin_alpha(const LimIn<T> &li, const VKeys<T, NQ> &kv, const T *sh, const T *u,
+template <typename T, int P, int NQ, typename KV>
+__device__ __forceinline__ bool lin_alpha(const LimIn<T> &li, const KV &kv, const T *sh, const T *u,
                                           int dmask, const T dataV0T[3], T *du) {
   constexpr int N = Dims<P>::N;
   const T third = T(1) / T(3), two3 = T(2) / T(3);
@@ -937,8 +1074,8 @@ __device__ __forceinline__ bool lin_alpha(const LimIn<T> &li, const VKeys<T, NQ>
 
 // lin_alpha with only u_0, u_1, u_2 given: the rows u_3.. of DM c are computed where the element
 // is limited (each row as lin_u computes it, so the results are the same).
-template <typename T, int P, int NQ>
-__device__ __forceinline__ bool lin_alpha_lazy(const LimIn<T> &li, const VKeys<T, NQ> &kv, const T *sh, T *u,
+template <typename T, int P, int NQ, typename KV>
+__device__ __forceinline__ bool lin_alpha_lazy(const LimIn<T> &li, const KV &kv, const T *sh, T *u,
                                                const T *c, int dmask, const T dataV0T[3], T *du) {
   constexpr int N = Dims<P>::N;
   const Tab<T, P> &tb = tab<T, P>();
@@ -996,13 +1133,15 @@ __device__ __forceinline__ void stage_op_tile(const Geo<T> g, const T *cin, cons
   uint64_t *bar = (uint64_t *)(smem + StageRows<T, P>::bar_offset(NT, 1, blockDim.x));
   const Tab<T, P> &tb = tab<T, P>();
   const int t = threadIdx.x, eb = blockDim.x, k0 = tile * eb, k = k0 + t;
-  pdl_trigger();
   const int Kp = g.Kp;
   const bool staged = k0 < g.K;                   // blocks beyond the elements only reset keys
   const bool first = sc.omega == 0.0;             // c^n has no part in this stage: not read
   constexpr int rC = 0, rC0 = N, rF = (MODE != 2) ? 2 * N : N, rV = rF + (EOP ? N * N : 2 * Q), rB = rV + 3 * R;
+  const bool vt = MODE != 0 && vt_on<T>();
+  const int vtOff = vt ? (int)StageRows<T, P>::bytes(NT, 1) : -1;
   if (staged) {
     if (t == 0) { mbar_init(bar, 1); mbar_fence_init(); }
+    if (vt) vt_reset(g, lo.nc, vtOff);
     __syncthreads();
     if (t == 0) {                                 // static rows before the dependency wait
       stage_expect<T>(bar, NT - (MODE != 2 && first ? N : 0), 1);
@@ -1023,7 +1162,9 @@ __device__ __forceinline__ void stage_op_tile(const Geo<T> g, const T *cin, cons
 #pragma unroll
   for (int n = 0; n < 3; ++n) nb[n] = active ? g.nbr[(size_t)n * Kp + k] : -1;
   int vid[3] = {0, 0, 0};
-  if (MODE != 0 && active) { vid[0] = g.V0T[k]; vid[1] = g.V0T[Kp + k]; vid[2] = g.V0T[2 * Kp + k]; }
+  if (MODE != 0 && active) load_vertices(g, k, vt, vid);
+  VtList vl{0, 0, 0};
+  if (vt && staged) vl = vt_list(g, tile);
   int ax = 0;
   T src[N];                                       // the source terms at this stage's time
   if constexpr (FXP) {                            // neighbours across inflow edges only
@@ -1042,6 +1183,7 @@ __device__ __forceinline__ void stage_op_tile(const Geo<T> g, const T *cin, cons
       if (!((ax >> (22 + n)) & 1)) nb[n] = -1;
   }
   pdl_wait();
+  pdl_trigger();
   if (MODE != 0) reset_next<T>(g, lo, k, nTiles < 0 ? -1 : tile, nTiles);
   if (!staged) return;
   if (t == 0) {                                   // state rows after it
@@ -1183,7 +1325,7 @@ __device__ __forceinline__ void stage_op_tile(const Geo<T> g, const T *cin, cons
       }
     }
   }
-  if (MODE != 0) scatter_quantities<T, NQ>(g, lo, qv, vid, active && ok, tile);
+  if (MODE != 0) scatter_quantities<T, NQ>(g, lo, qv, vid, active && ok, tile, vtOff, vl);
   if (bad) atomicOr(sc.flag, 1);
 }
 template <typename T, int P, int MODE, bool RHS, bool LIN, int VAR = kOpPlain>
@@ -1262,7 +1404,6 @@ __device__ __forceinline__ void stage_op_tile_mma(const Geo<float> g, const floa
   uint32_t *tslot = (uint32_t *)(mm + vmma::oTmem);
   const Tab<T, P> &tb = tab<T, P>();
   const int t = threadIdx.x, k0 = tile * kBlock, k = k0 + t;
-  pdl_trigger();
   const int Kp = g.Kp;
   const bool staged = k0 < g.K;
   constexpr int rC = 0, rF = N, rV = rF + 2 * Q, rB = rV + 3 * R;
@@ -1288,6 +1429,7 @@ __device__ __forceinline__ void stage_op_tile_mma(const Geo<float> g, const floa
   int vid[3] = {0, 0, 0};
   if (active) { vid[0] = g.V0T[k]; vid[1] = g.V0T[Kp + k]; vid[2] = g.V0T[2 * Kp + k]; }
   pdl_wait();
+  pdl_trigger();
   reset_next<T>(g, lo, k);
   if (!staged) return;
   const uint32_t tbase = *tslot;
@@ -1432,12 +1574,13 @@ k_limit_dot(const Geo<T> g, const T *cin, const T *c0, const T *tbuf, T *tout,
   uint64_t *bar = (uint64_t *)(smem + StageRows<T, P>::bar_offset(NT, 1, blockDim.x));
   const int t = threadIdx.x, k0 = blockIdx.x * kBlock, k = k0 + t;
   T *sh = (T *)(smem + StageRows<T, P>::bar_offset(NT, 1, blockDim.x) + 16);
-  pdl_trigger();
   const int Kp = g.Kp;
   const bool staged = k0 < g.K;
   constexpr int rT = 0, rB = N, rC0 = N + 4, rC = rC0 + N;
+  const int vtIn = (int)StageRows<T, P>::bytes(NT, 1), vtOff = vt_on<T>() ? vtIn + 2 * lo.nc * g.vtMax * (int)sizeof(T) : -1;
   if (staged) {
     if (t == 0) { mbar_init(bar, 1); mbar_fence_init(); }
+    if (vtOff >= 0) vt_reset(g, lo.nc, vtOff);
     __syncthreads();
     if (t == 0) {
       stage_expect<T>(bar, NT, 1);
@@ -1447,8 +1590,11 @@ k_limit_dot(const Geo<T> g, const T *cin, const T *c0, const T *tbuf, T *tout,
   }
   const bool active = k < g.K;
   int vid[3] = {0, 0, 0};
-  if (active) { vid[0] = g.V0T[k]; vid[1] = g.V0T[Kp + k]; vid[2] = g.V0T[2 * Kp + k]; }
+  if (active) load_vertices(g, k, true, vid);
+  VtList vl{0, 0, 0};
+  if (staged) vl = vt_list(g, blockIdx.x);
   pdl_wait();
+  pdl_trigger();
   reset_next<T>(g, lo, k);
   if (!staged) return;
   if (t == 0) {
@@ -1456,11 +1602,11 @@ k_limit_dot(const Geo<T> g, const T *cin, const T *c0, const T *tbuf, T *tout,
     stage_T(smem, rC0, c0, N, Kp, k0, bar);
     stage_T(smem, rC, cin, N, Kp, k0, bar);
   }
-  if (li.shift) load_shifts<T>(li.slots + slot_base(g, li.nc), li.nc, sh);
-  VKeys<T, NQ> kv;
-  load_vkeys<T, NQ>(g, li, vid, kv);
-  __syncthreads();
+  const PatchView<T> pv{(const T *)(smem + vtIn), g.vtMax, {vid[0], vid[1], vid[2]}};
+  load_patch<T, NQ>(g, li, blockIdx.x, vl, sh, vtIn);
   const bool ok = mbar_wait_bounded(bar, sc.flag);
+  int gid[3] = {0, 0, 0};   // vertex ids of the direct atomics (64-bit keys)
+  if (active && vtOff < 0) load_vertices(g, k, false, gid);
   T qv[NQ];
   bool bad = false;
   if (active && ok) {
@@ -1471,7 +1617,7 @@ k_limit_dot(const Geo<T> g, const T *cin, const T *c0, const T *tbuf, T *tout,
     for (int i = 0; i < N; ++i) { cT[i] = srow<T>(smem, rT + i)[t]; lim[i] = cT[i]; }
     const int dmask = (irow<T>(smem, NT, 0)[t] >> 9) & 7;
     const T nan3[3] = {T(NAN), T(NAN), T(NAN)};
-    limit_taylor<T, P, NQ, LT>(li, kv, sh, af, dmask, nan3, lim);
+    limit_taylor<T, P, NQ, LT>(li, pv, sh, af, dmask, nan3, lim);
     // Taylor mass correction M_corr = diag(1/diag(M_T)) M_T applied to (cT - lim); the packed
     // upper triangle is read once, row by row, and every row i of the product still sums its
     // terms in the order j = 0..N-1
@@ -1533,7 +1679,7 @@ k_limit_dot(const Geo<T> g, const T *cin, const T *c0, const T *tbuf, T *tout,
     for (int i = 0; i < N; ++i) { tout[(size_t)i * Kp + k] = cT2[i]; bad |= !finite_(cT2[i]); }
     centroid_quantities<T, P>(cT2, lo.type, qv);
   }
-  scatter_quantities<T, NQ>(g, lo, qv, vid, active && ok);
+  scatter_quantities<T, NQ>(g, lo, qv, vtOff < 0 ? gid : vid, active && ok, -1, vtOff, vl);
   if (bad) atomicOr(sc.flag, 1);
 }
 
@@ -1549,7 +1695,6 @@ k_limit(const Geo<T> g, const T *tbuf, T *__restrict__ out, const LimIn<T> li,
   uint64_t *bar = (uint64_t *)(smem + StageRows<T, P>::bar_offset(NT, 1, blockDim.x));
   const int t = threadIdx.x, k0 = blockIdx.x * kBlock, k = k0 + t;
   T *sh = (T *)(smem + StageRows<T, P>::bar_offset(NT, 1, blockDim.x) + 16);
-  pdl_trigger();
   if (k0 >= g.K) { pdl_wait(); return; }
   const int Kp = g.Kp;
   if (t == 0) { mbar_init(bar, 1); mbar_fence_init(); }
@@ -1561,13 +1706,14 @@ k_limit(const Geo<T> g, const T *tbuf, T *__restrict__ out, const LimIn<T> li,
   }
   const bool active = k < g.K;
   int vid[3] = {0, 0, 0};
-  if (active) { vid[0] = g.V0T[k]; vid[1] = g.V0T[Kp + k]; vid[2] = g.V0T[2 * Kp + k]; }
+  const int vtIn = (int)StageRows<T, P>::bytes(NT, 1);
+  if (active) load_vertices(g, k, true, vid);
+  const VtList vl = vt_list(g, blockIdx.x);
   pdl_wait();
+  pdl_trigger();
   if (t == 0) stage_T(smem, 0, tbuf, N, Kp, k0, bar);
-  if (li.shift) load_shifts<T>(li.slots + slot_base(g, li.nc), li.nc, sh);
-  VKeys<T, NQ> kv;
-  load_vkeys<T, NQ>(g, li, vid, kv);
-  __syncthreads();
+  const PatchView<T> pv{(const T *)(smem + vtIn), g.vtMax, {vid[0], vid[1], vid[2]}};
+  load_patch<T, NQ>(g, li, blockIdx.x, vl, sh, vtIn);
   T data[3] = {T(0), T(0), T(0)};
   if (g.cDV0T && active) {
     for (int m = 0; m < g.nTerms; ++m) {
@@ -1584,7 +1730,7 @@ k_limit(const Geo<T> g, const T *tbuf, T *__restrict__ out, const LimIn<T> li,
 #pragma unroll
   for (int i = 0; i < N; ++i) cT[i] = srow<T>(smem, i)[t];
   const int dmask = (irow<T>(smem, NT, 0)[t] >> 9) & 7;
-  limit_taylor<T, P, NQ, LT>(li, kv, sh, af, dmask, data, cT);
+  limit_taylor<T, P, NQ, LT>(li, pv, sh, af, dmask, data, cT);
   T c[N];
   from_taylor<T, P>(cT, af, c);
   bool bad = false;
@@ -1603,7 +1749,6 @@ k_to_taylor(const Geo<T> g, const T *c, T *__restrict__ tbuf, const LimOut<T> lo
   extern __shared__ __align__(128) unsigned char smem[];
   uint64_t *bar = (uint64_t *)(smem + StageRows<T, P>::bar_offset(NT, 0, blockDim.x));
   const int t = threadIdx.x, k0 = blockIdx.x * kBlock, k = k0 + t;
-  pdl_trigger();
   const int Kp = g.Kp;
   const bool staged = k0 < g.K;
   if (staged) {
@@ -1615,6 +1760,7 @@ k_to_taylor(const Geo<T> g, const T *c, T *__restrict__ tbuf, const LimOut<T> lo
   int vid[3] = {0, 0, 0};
   if (active) { vid[0] = g.V0T[k]; vid[1] = g.V0T[Kp + k]; vid[2] = g.V0T[2 * Kp + k]; }
   pdl_wait();
+  pdl_trigger();
   reset_next<T>(g, lo, k);
   if (!staged) return;
   if (t == 0) stage_T(smem, 0, c, N, Kp, k0, bar);
@@ -1647,19 +1793,20 @@ __device__ __forceinline__ void limit_dot_lin_tile(const Geo<T> g, const T *cin,
   // staged rows: cDot, then N(N-1) rows of Q_k or the 4 rows of B, then c^n and c^(s-1)
   const bool fly = g.mtOnTheFly != 0;
   const bool first = sc.omega == 0.0;   // c^n has no part in this stage: not read
-  // FP64 with stored rows and the global shift: the sums of products in fixed point
-  const bool fxOn = std::is_same_v<T, double> && !fly && li.shift && g.MTX != nullptr;
+  // FP64 with stored rows: the sums of products in fixed point
+  const bool fxOn = std::is_same_v<T, double> && !fly && g.MTX != nullptr;
   const int NT = StageRows<T, P>::limdot_lin_rows(fly);
   extern __shared__ __align__(128) unsigned char smem[];
   uint64_t *bar = (uint64_t *)(smem + StageRows<T, P>::bar_offset(NT, 1, blockDim.x));
   const int t = threadIdx.x, k0 = tile * kBlock, k = k0 + t;
   T *sh = (T *)(smem + StageRows<T, P>::bar_offset(NT, 1, blockDim.x) + 16);
-  pdl_trigger();
   const int Kp = g.Kp;
   const bool staged = k0 < g.K;
   const int rD = 0, rQ = N, rC0 = NT - 2 * N, rC = rC0 + N;
+  const int vtIn = (int)StageRows<T, P>::bytes(NT, 1), vtOff = vt_on<T>() ? vtIn + 2 * g.vtMax * (int)sizeof(T) : -1;
   if (staged) {
     if (t == 0) { mbar_init(bar, 1); mbar_fence_init(); }
+    if (vtOff >= 0) vt_reset(g, 1, vtOff);
     __syncthreads();
     if (t == 0) {
       stage_expect<T>(bar, NT - (first ? N : 0), 1);
@@ -1670,10 +1817,13 @@ __device__ __forceinline__ void limit_dot_lin_tile(const Geo<T> g, const T *cin,
   }
   const bool active = k < g.K;
   int vid[3] = {0, 0, 0};
-  if (active) { vid[0] = g.V0T[k]; vid[1] = g.V0T[Kp + k]; vid[2] = g.V0T[2 * Kp + k]; }
+  if (active) load_vertices(g, k, true, vid);
+  VtList vl{0, 0, 0};
+  if (staged) vl = vt_list(g, tile);
   int mx = -1;
   if (fxOn && active) mx = g.mtE[k];
   pdl_wait();
+  pdl_trigger();
   reset_next<T>(g, lo, k, nTiles < 0 ? -1 : tile, nTiles);
   if (!staged) return;
   if (t == 0) {
@@ -1681,11 +1831,11 @@ __device__ __forceinline__ void limit_dot_lin_tile(const Geo<T> g, const T *cin,
     if (!first) stage_T(smem, rC0, c0, N, Kp, k0, bar);
     stage_T(smem, rC, cin, N, Kp, k0, bar);
   }
-  if (li.shift) load_shifts<T>(li.slots + slot_base(g, li.nc, tile), li.nc, sh);
-  VKeys<T, NQ> kv;
-  load_vkeys<T, NQ>(g, li, vid, kv);
-  __syncthreads();
+  const PatchView<T> pv{(const T *)(smem + vtIn), g.vtMax, {vid[0], vid[1], vid[2]}};
+  load_patch<T, NQ>(g, li, tile, vl, sh, vtIn);
   const bool ok = mbar_wait_bounded(bar, sc.flag);
+  int gid[3] = {0, 0, 0};   // vertex ids of the direct atomics (64-bit keys)
+  if (active && vtOff < 0) load_vertices(g, k, false, gid);
   T q0 = T(0);
   bool bad = false;
   if (active && ok) {
@@ -1696,16 +1846,14 @@ __device__ __forceinline__ void limit_dot_lin_tile(const Geo<T> g, const T *cin,
     if constexpr (std::is_same_v<T, double>)
       if (fxOn) {
         T lo3[3], hi3[3];
-#pragma unroll
-        for (int n = 0; n < 3; ++n) { lo3[n] = vkey_inv<T>(kv.v[0][0][n]); hi3[n] = vkey_inv<T>(kv.v[0][1][n]); }
-        limited = fx::linear_cdot_limit<P>(fx_tab<P>(), lo3, hi3, sh[0], sh[1], (const Dig *)srow<T>(smem, rQ) + t,
-                                           kBlock, mx, cd);
+        patch_extremes(li, pv, sh, lo3, hi3);
+        limited = fx::linear_cdot_limit<P>(fx_tab<P>(), lo3, hi3, (const Dig *)srow<T>(smem, rQ) + t, kBlock, mx, cd);
       }
     if (!limited) {
     lin_u3<T, P>(cd, u);
     const int dmask = (irow<T>(smem, NT, 0)[t] >> 9) & 7;
     const T nan3[3] = {T(NAN), T(NAN), T(NAN)};
-    if (lin_alpha_lazy<T, P, NQ>(li, kv, sh, u, cd, dmask, nan3, du)) {
+    if (lin_alpha_lazy<T, P, NQ>(li, pv, sh, u, cd, dmask, nan3, du)) {
       if (fly) {
         const Affine<T> af = affine_from<T>(srow<T>(smem, rQ)[t], srow<T>(smem, rQ + 1)[t],
                                             srow<T>(smem, rQ + 2)[t], srow<T>(smem, rQ + 3)[t]);
@@ -1757,7 +1905,7 @@ __device__ __forceinline__ void limit_dot_lin_tile(const Geo<T> g, const T *cin,
     for (int i = 0; i < N; ++i) { out[(size_t)i * Kp + k] = cnew[i]; bad |= !finite_(cnew[i]); }
     q0 = lin_mean<T, P>(cnew);
   }
-  scatter_quantities<T, NQ>(g, lo, &q0, vid, active && ok, tile);
+  scatter_quantities<T, NQ>(g, lo, &q0, vtOff < 0 ? gid : vid, active && ok, tile, vtOff, vl);
   if (bad) atomicOr(sc.flag, 1);
 }
 template <typename T, int P>
@@ -1767,20 +1915,19 @@ k_limit_dot_lin(const Geo<T> g, const T *cin, const T *c0, const T *tbuf,
   limit_dot_lin_tile<T, P>(g, cin, c0, tbuf, out, li, lo, sc, blockIdx.x);
 }
 
-// One element's coefficients limited in place.
-template <typename T, int P>
-__device__ __forceinline__ void limit_lin_element(const LimIn<T> &li, const VKeys<T, 1> &kv, const T *sh, int dmask,
+// One element's coefficients limited in place (FX: FP64 sums in fixed point).
+template <typename T, int P, bool FX, typename KV>
+__device__ __forceinline__ void limit_lin_element(const LimIn<T> &li, const KV &kv, const T *sh, int dmask,
                                                   const T data[3], T *c) {
   constexpr int N = Dims<P>::N, NQ = 1;
   const Tab<T, P> &tb = tab<T, P>();
   T u[N], du[N];
   bool limited = false;   // c is done in fixed point
-  if constexpr (std::is_same_v<T, double>)
-    if (li.shift) {
+  if constexpr (FX && std::is_same_v<T, double>)
+    {
       T lo3[3], hi3[3];
-#pragma unroll
-      for (int n = 0; n < 3; ++n) { lo3[n] = vkey_inv<T>(kv.v[0][0][n]); hi3[n] = vkey_inv<T>(kv.v[0][1][n]); }
-      limited = fx::linear_limit<P>(fx_tab<P>(), lo3, hi3, sh[0], sh[1], dmask, data, c);
+      patch_extremes(li, kv, sh, lo3, hi3);
+      limited = fx::linear_limit<P>(fx_tab<P>(), lo3, hi3, dmask, data, c);
     }
   if (!limited) {
   lin_u3<T, P>(c, u);
@@ -1810,12 +1957,11 @@ __device__ __forceinline__ void limit_lin_tile(const Geo<T> g, const T *cbuf, T 
   constexpr int N = Dims<P>::N, NQ = 1;
   __shared__ T sh[2];
   const int t = threadIdx.x, k = tile * kBlock + t;
-  pdl_trigger();
   const bool active = k < g.K;
   const int Kp = g.Kp;
   int vid[3] = {0, 0, 0}, dmask = 0;
   if (active) {
-    vid[0] = g.V0T[k]; vid[1] = g.V0T[Kp + k]; vid[2] = g.V0T[2 * Kp + k];
+    load_vertices(g, k, true, vid);
     dmask = (g.code[k] >> 9) & 7;
   }
   T data[3] = {T(0), T(0), T(0)};
@@ -1826,16 +1972,17 @@ __device__ __forceinline__ void limit_lin_tile(const Geo<T> g, const T *cbuf, T 
       for (int n = 0; n < 3; ++n) data[n] += gm * g.cDV0T[((size_t)m * 3 + n) * Kp + k];
     }
   }
+  const VtList vl = vt_list(g, tile);
   pdl_wait();
-  if (li.shift) load_shifts<T>(li.slots + slot_base(g, li.nc, tile), li.nc, sh);
+  pdl_trigger();
   T c[N];
 #pragma unroll
   for (int i = 0; i < N; ++i) c[i] = active ? cbuf[(size_t)i * Kp + k] : T(0);
-  VKeys<T, NQ> kv;
-  load_vkeys<T, NQ>(g, li, vid, kv);
-  __syncthreads();
+  extern __shared__ __align__(128) unsigned char smem[];
+  const PatchView<T> pv{(const T *)smem, g.vtMax, {vid[0], vid[1], vid[2]}};
+  load_patch<T, NQ>(g, li, tile, vl, sh, 0);
   if (!active) return;
-  limit_lin_element<T, P>(li, kv, sh, dmask, data, c);
+  limit_lin_element<T, P, true>(li, pv, sh, dmask, data, c);
   bool bad = false;
 #pragma unroll
   for (int i = 0; i < N; ++i) { out[(size_t)i * Kp + k] = c[i]; bad |= !finite_(c[i]); }
@@ -1855,12 +2002,12 @@ __global__ void __launch_bounds__(kBlock)
 k_mean_lin(const Geo<T> g, const T *c, const LimOut<T> lo, T *__restrict__ meanOut) {
   constexpr int N = Dims<P>::N;
   const int t = threadIdx.x, k = blockIdx.x * kBlock + t;
-  pdl_trigger();
   const bool active = k < g.K;
   const int Kp = g.Kp;
   int vid[3] = {0, 0, 0};
   if (active) { vid[0] = g.V0T[k]; vid[1] = g.V0T[Kp + k]; vid[2] = g.V0T[2 * Kp + k]; }
   pdl_wait();
+  pdl_trigger();
   reset_next<T>(g, lo, k);
   T q0 = T(0);
   if (active) {
@@ -1918,7 +2065,6 @@ k_op_fused(const Geo<T> g, const T *x, int limitIn, T *xLout,
   T *sh = (T *)(smem + StageRows<T, P>::bar_offset(NT, 1, blockDim.x) + 16);
   const Tab<T, P> &tb = tab<T, P>();
   const int t = threadIdx.x, k0 = blockIdx.x * kBlock, k = k0 + t;
-  pdl_trigger();
   const int Kp = g.Kp;
   const bool staged = k0 < g.K;
   constexpr int rC = 0, rC0 = N, rF = (MODE != 2) ? 2 * N : N, rV = rF + 2 * Q;
@@ -1947,6 +2093,7 @@ k_op_fused(const Geo<T> g, const T *x, int limitIn, T *xLout,
     v3[n] = nb[n] >= 0 ? g.V0T[(size_t)np * Kp + nb[n]] : 0;
   }
   pdl_wait();
+  pdl_trigger();
   reset_next<T>(g, lo, k);
   if (!staged) return;
   if (t == 0) {

@@ -103,7 +103,7 @@ struct Sum {
   }
 };
 __device__ __forceinline__ long long shr(long long x, int s) {   // x >> s for s of either sign
-  return s >= 0 ? x >> min(s, 63) : x << -s;
+  return s >= 0 ? x >> min(s, 63) : x << min(-s, 63);
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -190,18 +190,18 @@ __device__ __forceinline__ bool element_cdot(const FxTab<P> &tb, const Dig *sA, 
 }
 
 // ---------------------------------------------------------------------------------------------
-// The linear limiter's factor (vertex_alpha_1div) for u_0, u_1, u_2 given as u[i] 2^(uu[i]), in
-// integers of one unit, 2^(G - 1082), that holds the global shift, the patch extremes and u: the
-// differences, comparisons and cross products are exact, and the reference's shift of the patch
-// extremes (a - s) + s rounds (s - a) to 53 bits as FP64 does.  The unit is
-// at most the spacing that the shift leaves in FP64, and usually 2^-6 of it.
+// The linear limiter's factor (vertex_alpha_1div) for u_0, u_1, u_2 given as u[i] 2^(uu[i]) and the
+// patch extremes (shifted), in integers of one unit, 2^(G - 1082), that holds them all: the
+// differences, comparisons and cross products are exact.  G is the largest exponent among the
+// extremes and u, so the unit is 2^-60 of the largest value, where FP64 rounds at 2^-53 of each.
 // Returns 0: not limited, 1: limited by alpha, -1: left to FP64.
-__device__ __forceinline__ int linear_alpha(const double lo[3], const double hi[3], double shPos, double shNeg,
-                                            int dmask, const double data[3], const long long u[3], const int uu[3],
-                                            double &alpha) {
-  const int S = max(expo(shPos), expo(shNeg));
+__device__ __forceinline__ int linear_alpha(const double lo[3], const double hi[3], int dmask, const double data[3],
+                                            const long long u[3], const int uu[3], double &alpha) {
+  int S = 1000;                                   // the tolerance 1e-8 (exponent 996) fits the unit
+#pragma unroll
+  for (int n = 0; n < 3; ++n) S = max(S, max(expo(lo[n]), expo(hi[n])));
+  if (S > kExpHi) return -1;
   int G = S;
-  if (S < 1023 || S > kExpHi) return -1;          // the shifts are at least 1
 #pragma unroll
   for (int i = 0; i < 3; ++i) {
     const long long m = u[i] < 0 ? ~u[i] : u[i];
@@ -224,22 +224,13 @@ __device__ __forceinline__ int linear_alpha(const double lo[3], const double hi[
 #pragma unroll
     for (int n = 0; n < 3; ++n) dat[n] = fix<60>(data[n], G);
   }
-  const long long sP = fix<60>(shPos, G), sN = fix<60>(shNeg, G), tol3 = 3 * fix<60>(1.e-8, G);
+  const long long tol3 = 3 * fix<60>(1.e-8, G);
   const long long dV3[3] = {-(U[1] + U[2]), 2 * U[1] - U[2], 2 * U[2] - U[1]};
   unsigned long long bn = 0, bd = 1;
   bool any = false;
 #pragma unroll
   for (int n = 0; n < 3; ++n) {
-    const double a = lo[n], b = hi[n];
-    if (expo(a) > S || expo(b) > S) return -1;    // an extreme that is not a number
-    // t = s - a >= 1: to the nearest multiple of its 53-bit spacing, ties to even
-    auto shifted = [](long long t) {
-      const int k = max(11 - __clzll(t), 0);
-      const unsigned one = 1u << k, up = ((one >> 1) + (((unsigned)t >> k) & 1u) - 1u) & (one - 1u);
-      return (t + (long long)up) & ~(long long)(one - 1u);
-    };
-    long long mn = sN - shifted(sN - fix<60>(a, G));
-    long long mx = shifted(sP + fix<60>(b, G)) - sP;
+    long long mn = fix<60>(lo[n], G), mx = fix<60>(hi[n], G);
     if ((dmask >> n) & 1) { mn = min(mn, dat[n]); mx = max(mx, dat[n]); }
     const long long dMin3 = 3 * (mn - U[0]), dMax3 = 3 * (mx - U[0]);
     long long num = 0, den = 1;
@@ -276,12 +267,12 @@ __device__ __forceinline__ void reference_derivatives(const FxTab<P> &tb, const 
 // sQ: digits of Q_k with column j scaled by 2^(eDM_j), row i (N-1) + (j-1), stride st; qx: the
 // exponent of its largest row sum (negative: not in fixed point).  False: left to FP64.
 template <int P>
-__device__ __forceinline__ bool linear_cdot_limit(const FxTab<P> &tb, const double lo[3], const double hi[3], double shPos,
-                                                  double shNeg, const Dig *sQ, int st, int qx, double *cd) {
+__device__ __forceinline__ bool linear_cdot_limit(const FxTab<P> &tb, const double lo[3], const double hi[3],
+                                                  const Dig *sQ, int st, int qx, double *cd) {
   constexpr int N = Dims<P>::N;
   int E = max_expo<N>(cd);
   if (qx < 0 || E > kExpHi) return false;
-  E = max(E, kExpLo);                              // below 2^-457 of the shift's 1: zero
+  E = max(E, kExpLo);                              // what is below 2^-457 counts as zero
   Dig d[N];
 #pragma unroll
   for (int j = 0; j < N; ++j) d[j] = digits_of(cd[j], E);
@@ -290,7 +281,7 @@ __device__ __forceinline__ bool linear_cdot_limit(const FxTab<P> &tb, const doub
   const int uu[3] = {E - 1022 + tb.eDM[0] - 58, E - 1022 + tb.eDM[1] - 58, E - 1022 + tb.eDM[2] - 58};
   double alpha;
   const double none[3] = {0.0, 0.0, 0.0};
-  const int how = linear_alpha(lo, hi, shPos, shNeg, 0, none, u, uu, alpha);
+  const int how = linear_alpha(lo, hi, 0, none, u, uu, alpha);
   if (how <= 0) return how == 0;
   reference_derivatives<P, 3, N>(tb, d, u);
   const Dig om = digits_of(1.0 - alpha, 1023);   // (1 - alpha) 2^56
@@ -320,8 +311,8 @@ __device__ __forceinline__ bool linear_cdot_limit(const FxTab<P> &tb, const doub
 // Solution limiting of c in place (limit_lin_tile): where limited, the linear Taylor polynomial
 // (u_0, alpha u_1, alpha u_2) in the modal basis.  False: left to FP64.
 template <int P>
-__device__ __forceinline__ bool linear_limit(const FxTab<P> &tb, const double lo[3], const double hi[3], double shPos, double shNeg,
-                                             int dmask, const double data[3], double *c) {
+__device__ __forceinline__ bool linear_limit(const FxTab<P> &tb, const double lo[3], const double hi[3], int dmask,
+                                             const double data[3], double *c) {
   constexpr int N = Dims<P>::N;
   int E = max_expo<N>(c);
   if (E > kExpHi) return false;
@@ -333,7 +324,7 @@ __device__ __forceinline__ bool linear_limit(const FxTab<P> &tb, const double lo
   reference_derivatives<P, 0, 3>(tb, d, u);
   const int uu[3] = {E - 1022 + tb.eDM[0] - 58, E - 1022 + tb.eDM[1] - 58, E - 1022 + tb.eDM[2] - 58};
   double alpha;
-  const int how = linear_alpha(lo, hi, shPos, shNeg, dmask, data, u, uu, alpha);
+  const int how = linear_alpha(lo, hi, dmask, data, u, uu, alpha);
   if (how <= 0) return how == 0;
   const Dig al = digits_of(alpha, 1023);
   Dig w[3] = {digits(u[0]), {0, 0}, {0, 0}};

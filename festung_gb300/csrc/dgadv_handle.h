@@ -27,6 +27,7 @@ void transport_release(dgadv_handle *h);
 // precisions, implicit handles, or with DGADV_OPT_ELEMENT_OPERATOR = 0).
 int refresh_element_operator(dgadv_handle *h);
 constexpr int kBlock = 128;       // elements per CTA (one thread per element)
+constexpr int kMaxBlockVertices = 3 * kBlock;   // longest vertex list a block of elements can have
 constexpr int kSlotCopies = 32;   // copies of the global min / max slots (atomics spread over them)
 constexpr int kGridBarBytes = 8192;   // state of the persistent step's grid barrier
 constexpr int kMaxLinkedParts = 4;    // handles in one linked step (a primary and three more)
@@ -42,6 +43,9 @@ struct dgadv_handle {
   // device arrays (element type depends on prec)
   void *F = nullptr, *Vn = nullptr, *Bm = nullptr, *MT = nullptr, *rhs = nullptr, *cDV0T = nullptr;
   int *nbr = nullptr, *code = nullptr, *V0T = nullptr, *vptr = nullptr, *vidx = nullptr, *perm = nullptr;
+  int *vtPtr = nullptr, *vtIdx = nullptr;   // vertices of each block of kBlock elements (Geo)
+  unsigned short *vtLoc = nullptr;
+  int vtMax = 0;
   int nInst = 1;                       // ensembles: instances (each its own limiter extremes)
   int *instOf = nullptr;               // ensembles: instance of each block of kBlock elements
   std::vector<int> instStart;          // first element of each instance (caller order), + K

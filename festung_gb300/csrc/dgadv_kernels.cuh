@@ -82,6 +82,12 @@ template <typename T> struct Geo {
   int mtOnTheFly;    // forward kernels rebuild the Taylor mass correction from B and Gr instead
                      // of reading MT (the limiter adjoint still reads MT)
   const int *V0T;    // 3 x Kp   vertex ids
+  // vertices of each block of 128 elements: list vtIdx[vtPtr[b] .. vtPtr[b + 1]) (ascending) and every
+  // element's positions in its block's list (3 x Kp); vtMax: the longest list (0 without
+  // a limiter)
+  const int *vtPtr, *vtIdx;
+  const unsigned short *vtLoc;
+  int vtMax;
   const int *vptr;   // numV+1   CSR vertex -> elements
   const int *vidx;
   const T *rhs;      // nTerms x N x Kp   (L - K_D - K_N)_m / detJ

@@ -164,6 +164,7 @@ static Geo<T> make_geo(const dgadv_handle *h) {
   g.AopX = (const Dig *)h->AopX; g.VnX = (const Dig *)h->VnX; g.MTX = (const Dig *)h->MTX;
   g.aopE = h->aopE; g.mtE = h->mtE;
   g.rhsM = h->nTerms > 0 ? (const T *)h->rhsM : nullptr;
+  g.vtPtr = h->vtPtr; g.vtIdx = h->vtIdx; g.vtLoc = h->vtLoc; g.vtMax = h->vtMax;
   return g;
 }
 
@@ -283,14 +284,29 @@ static cudaError_t copy_state(dgadv_handle *h, void *dst, const void *src, size_
   return cudaGetLastError();
 }
 
+// Shared memory of `n` block-local vertex tables (extremes read, or keys gathered), after a kernel's
+// staged rows; with blocks of another size than kBlock the tables are not used.
+template <typename T> static size_t vt_bytes(const dgadv_handle *h, int n, int block = kBlock) {
+  return block == kBlock ? (size_t)n * 2 * h->nc * h->vtMax * sizeof(T) : 0;
+}
+// ... of a producer's key table (32-bit keys: vt_on), beside n tables of extremes
+template <typename T> static size_t vt_key_bytes(const dgadv_handle *h, int n, int block = kBlock) {
+  return vt_bytes<T>(h, n + (sizeof(typename KeyOf<T>::type) == 4 ? 1 : 0), block);
+}
+// ... at most, for the kernels' opt-in sizes
+template <typename T, int P> constexpr size_t vt_most(int n) {
+  return (size_t)n * 2 * NCQ<P>::value * kMaxBlockVertices * sizeof(T);
+}
+
 // Opt-in shared memory sizes of the staged kernels of one (precision, degree).
 template <typename T, int P, bool FUSED>
 static cudaError_t set_smem_attributes() {
   using SR = StageRows<T, P>;
   cudaError_t e = cudaSuccess;
-  auto set = [&](const void *f, size_t b) {
+  auto set0 = [&](const void *f, size_t b) {
     if (e == cudaSuccess) e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)b);
   };
+  auto set = [&](const void *f, size_t b) { set0(f, b + vt_most<T, P>(2)); };   // with both vertex tables
   set((const void *)k_stage_op<T, P, 0, true, false>, SR::bytes(SR::op(0, false), 1));
   set((const void *)k_stage_op<T, P, 0, false, false>, SR::bytes(SR::op(0, false), 1));
   set((const void *)k_stage_op<T, P, 1, true, false>, SR::bytes(SR::op(1, false), 1));
@@ -322,19 +338,19 @@ static cudaError_t set_smem_attributes() {
     set((const void *)k_stage_op<T, P, 2, false, true, true>, SR::bytes(SR::op(2, true), 1));
   }
   if constexpr (FUSED) {
-    set((const void *)k_op_fused<T, P, 1, true>, SR::bytes(SR::op(1, true), 1));
-    set((const void *)k_op_fused<T, P, 1, false>, SR::bytes(SR::op(1, true), 1));
-    set((const void *)k_op_fused<T, P, 2, true>, SR::bytes(SR::op(2, true), 1));
-    set((const void *)k_op_fused<T, P, 2, false>, SR::bytes(SR::op(2, true), 1));
+    set0((const void *)k_op_fused<T, P, 1, true>, SR::bytes(SR::op(1, true), 1));
+    set0((const void *)k_op_fused<T, P, 1, false>, SR::bytes(SR::op(1, true), 1));
+    set0((const void *)k_op_fused<T, P, 2, true>, SR::bytes(SR::op(2, true), 1));
+    set0((const void *)k_op_fused<T, P, 2, false>, SR::bytes(SR::op(2, true), 1));
   }
   set((const void *)k_limit_dot<T, P, 1>, SR::bytes(SR::limdot(), 1));
   set((const void *)k_limit_dot<T, P, 2>, SR::bytes(SR::limdot(), 1));
   set((const void *)k_limit<T, P, 1>, SR::bytes(SR::lim(), 1));
   set((const void *)k_limit<T, P, 2>, SR::bytes(SR::lim(), 1));
-  set((const void *)k_to_taylor<T, P>, SR::bytes(SR::totaylor(), 0));
+  set0((const void *)k_to_taylor<T, P>, SR::bytes(SR::totaylor(), 0));
   if constexpr (std::is_same_v<T, float> && P >= 2) {
-    set((const void *)k_stage_op_mma<P, true>, MmaSmem<P>::bytes(true));
-    set((const void *)k_stage_op_mma<P, false>, MmaSmem<P>::bytes(false));
+    set0((const void *)k_stage_op_mma<P, true>, MmaSmem<P>::bytes(true));
+    set0((const void *)k_stage_op_mma<P, false>, MmaSmem<P>::bytes(false));
   }
   return e;
 }
@@ -364,6 +380,7 @@ static cudaError_t launch_step(dgadv_handle *h, double t0, double tau) {
   const int gridK = (h->K + kBlock - 1) / kBlock;
   // the stage operator's elements per block (DGADV_OPT_OP_BLOCK; one thread per element)
   const int eb = h->opBlock, gridOp = (std::max(h->K, h->numV) + eb - 1) / eb;
+  const size_t vtOp = vt_key_bytes<T>(h, 0, eb);
   double omega[3], cst[3];
   const int S = rk_table(h->ordRK, omega, cst);
   T *cA = (T *)h->cA, *cB = (T *)h->cB, *tb = (T *)h->tbuf;
@@ -413,19 +430,19 @@ static cudaError_t launch_step(dgadv_handle *h, double t0, double tau) {
     if (viaMma) {
     } else if (mode == 2) {
       if (lin) {
-        if (rhs) launch_kb(h, stage_kernel<T, P, 2, true, true>(h), gridOp, eb, SR::bytes(stage_rows<T, P>(h, 2, true, true), 1, eb), g, in, cn, cdB, lo1, sc);
-        else launch_kb(h, stage_kernel<T, P, 2, false, true>(h), gridOp, eb, SR::bytes(stage_rows<T, P>(h, 2, true, false), 1, eb), g, in, cn, cdB, lo1, sc);
+        if (rhs) launch_kb(h, stage_kernel<T, P, 2, true, true>(h), gridOp, eb, SR::bytes(stage_rows<T, P>(h, 2, true, true), 1, eb) + vtOp, g, in, cn, cdB, lo1, sc);
+        else launch_kb(h, stage_kernel<T, P, 2, false, true>(h), gridOp, eb, SR::bytes(stage_rows<T, P>(h, 2, true, false), 1, eb) + vtOp, g, in, cn, cdB, lo1, sc);
       } else {
-        if (rhs) launch_kb(h, stage_kernel<T, P, 2, true, false>(h), gridOp, eb, SR::bytes(stage_rows<T, P>(h, 2, false, true), 1, eb), g, in, cn, cdB, lo1, sc);
-        else launch_kb(h, stage_kernel<T, P, 2, false, false>(h), gridOp, eb, SR::bytes(stage_rows<T, P>(h, 2, false, false), 1, eb), g, in, cn, cdB, lo1, sc);
+        if (rhs) launch_kb(h, stage_kernel<T, P, 2, true, false>(h), gridOp, eb, SR::bytes(stage_rows<T, P>(h, 2, false, true), 1, eb) + vtOp, g, in, cn, cdB, lo1, sc);
+        else launch_kb(h, stage_kernel<T, P, 2, false, false>(h), gridOp, eb, SR::bytes(stage_rows<T, P>(h, 2, false, false), 1, eb) + vtOp, g, in, cn, cdB, lo1, sc);
       }
     } else {
       if (lin) {
-        if (rhs) launch_kb(h, stage_kernel<T, P, 1, true, true>(h), gridOp, eb, SR::bytes(stage_rows<T, P>(h, 1, true, true), 1, eb), g, in, cn, yB, lo1, sc);
-        else launch_kb(h, stage_kernel<T, P, 1, false, true>(h), gridOp, eb, SR::bytes(stage_rows<T, P>(h, 1, true, false), 1, eb), g, in, cn, yB, lo1, sc);
+        if (rhs) launch_kb(h, stage_kernel<T, P, 1, true, true>(h), gridOp, eb, SR::bytes(stage_rows<T, P>(h, 1, true, true), 1, eb) + vtOp, g, in, cn, yB, lo1, sc);
+        else launch_kb(h, stage_kernel<T, P, 1, false, true>(h), gridOp, eb, SR::bytes(stage_rows<T, P>(h, 1, true, false), 1, eb) + vtOp, g, in, cn, yB, lo1, sc);
       } else {
-        if (rhs) launch_kb(h, stage_kernel<T, P, 1, true, false>(h), gridOp, eb, SR::bytes(stage_rows<T, P>(h, 1, false, true), 1, eb), g, in, cn, yB, lo1, sc);
-        else launch_kb(h, stage_kernel<T, P, 1, false, false>(h), gridOp, eb, SR::bytes(stage_rows<T, P>(h, 1, false, false), 1, eb), g, in, cn, yB, lo1, sc);
+        if (rhs) launch_kb(h, stage_kernel<T, P, 1, true, false>(h), gridOp, eb, SR::bytes(stage_rows<T, P>(h, 1, false, true), 1, eb) + vtOp, g, in, cn, yB, lo1, sc);
+        else launch_kb(h, stage_kernel<T, P, 1, false, false>(h), gridOp, eb, SR::bytes(stage_rows<T, P>(h, 1, false, false), 1, eb) + vtOp, g, in, cn, yB, lo1, sc);
       }
     }
     prof_mark(h, -1);
@@ -434,22 +451,22 @@ static cudaError_t launch_step(dgadv_handle *h, double t0, double tau) {
       const LimOut<T> lo2 = lim_out<T>(h);
       ++h->limPass;
       prof_mark(h, 1);
-      if (lin) launch_k(h, k_limit_dot_lin<T, P>, grid, SR::bytes(SR::limdot_lin_rows(h->mtOnTheFly), 1), g, (const T *)in, (const T *)cn, (const T *)cdB, yB, lim_in<T>(lo1, h), lo2, sc);
+      if (lin) launch_k(h, k_limit_dot_lin<T, P>, grid, SR::bytes(SR::limdot_lin_rows(h->mtOnTheFly), 1) + vt_key_bytes<T>(h, 1), g, (const T *)in, (const T *)cn, (const T *)cdB, yB, lim_in<T>(lo1, h), lo2, sc);
       else if (h->limType == DGADV_LIM_STRICT)
-        launch_k(h, k_limit_dot<T, P, 2>, grid, SR::bytes(SR::limdot(), 1), g, in, cn, (const T *)cdB, yB, lim_in<T>(lo1, h), lo2, sc);
+        launch_k(h, k_limit_dot<T, P, 2>, grid, SR::bytes(SR::limdot(), 1) + vt_key_bytes<T>(h, 1), g, in, cn, (const T *)cdB, yB, lim_in<T>(lo1, h), lo2, sc);
       else
-        launch_k(h, k_limit_dot<T, P, 1>, grid, SR::bytes(SR::limdot(), 1), g, in, cn, (const T *)cdB, yB, lim_in<T>(lo1, h), lo2, sc);
+        launch_k(h, k_limit_dot<T, P, 1>, grid, SR::bytes(SR::limdot(), 1) + vt_key_bytes<T>(h, 1), g, in, cn, (const T *)cdB, yB, lim_in<T>(lo1, h), lo2, sc);
       prof_mark(h, -1);
       loS = lo2;
     }
     // the adjoint's recomputation wants the limiter inputs only: c^(n+1) is not written
     if (h->stepRecordsOnly && s == S - 1) break;
     prof_mark(h, 2);
-    if (lin) launch_k(h, k_limit_lin<T, P>, gridK, (size_t)0, g, (const T *)yB, out, lim_in<T>(loS, h), scBC);
+    if (lin) launch_k(h, k_limit_lin<T, P>, gridK, vt_bytes<T>(h, 1), g, (const T *)yB, out, lim_in<T>(loS, h), scBC);
     else if (h->limType == DGADV_LIM_STRICT)
-      launch_k(h, k_limit<T, P, 2>, grid, SR::bytes(SR::lim(), 1), g, (const T *)yB, out, lim_in<T>(loS, h), scBC);
+      launch_k(h, k_limit<T, P, 2>, grid, SR::bytes(SR::lim(), 1) + vt_bytes<T>(h, 1), g, (const T *)yB, out, lim_in<T>(loS, h), scBC);
     else
-      launch_k(h, k_limit<T, P, 1>, grid, SR::bytes(SR::lim(), 1), g, (const T *)yB, out, lim_in<T>(loS, h), scBC);
+      launch_k(h, k_limit<T, P, 1>, grid, SR::bytes(SR::lim(), 1) + vt_bytes<T>(h, 1), g, (const T *)yB, out, lim_in<T>(loS, h), scBC);
     prof_mark(h, -1);
   }
   if (S == 1 && nRun == 1 && (const T *)dst == cn && !h->stepRecordsOnly) return copy_state(h, dst, cA, (size_t)h->N * h->Kp * sizeof(T));
@@ -500,7 +517,7 @@ static cudaError_t launch_step_fused(dgadv_handle *h, double t0, double tau, boo
     const LimOut<T> lo2 = lim_out<T>(h);
     ++h->limPass;
     prof_mark(h, 1);
-    launch_k(h, k_limit_dot_lin<T, P>, grid, SR::bytes(SR::limdot_lin_rows(h->mtOnTheFly), 1), g, (const T *)xL, (const T *)cnL,
+    launch_k(h, k_limit_dot_lin<T, P>, grid, SR::bytes(SR::limdot_lin_rows(h->mtOnTheFly), 1) + vt_key_bytes<T>(h, 1), g, (const T *)xL, (const T *)cnL,
              (const T *)tb, outRaw, lim_in<T>(lo1, h), lo2, sc);
     prof_mark(h, -1);
   }
@@ -514,7 +531,7 @@ static cudaError_t launch_finalize_fused(dgadv_handle *h) {
   StageScalars sc{};
   sc.flag = h->flag;
   prof_mark(h, 2);
-  launch_k(h, k_limit_lin<T, P>, gridK, (size_t)0, g, (const T *)h->cR, (T *)h->cn,
+  launch_k(h, k_limit_lin<T, P>, gridK, vt_bytes<T>(h, 1), g, (const T *)h->cR, (T *)h->cn,
            lim_in_pass<T>(h, h->limPass - 1), sc);
   prof_mark(h, -1);
   return cudaGetLastError();
@@ -533,13 +550,13 @@ static cudaError_t launch_limit_state(dgadv_handle *h, double t) {
   if (h->limType == DGADV_LIM_LINEAR) {
     const int gridK = (h->K + kBlock - 1) / kBlock;
     launch_k(h, k_mean_lin<T, P>, grid, (size_t)0, g, (const T *)h->cn, lo, (T *)nullptr);
-    launch_k(h, k_limit_lin<T, P>, gridK, (size_t)0, g, (const T *)h->cn, (T *)h->cn, lim_in<T>(lo, h), sc);
+    launch_k(h, k_limit_lin<T, P>, gridK, vt_bytes<T>(h, 1), g, (const T *)h->cn, (T *)h->cn, lim_in<T>(lo, h), sc);
   } else {
     launch_k(h, k_to_taylor<T, P>, grid, SR::bytes(SR::totaylor(), 0), g, (const T *)h->cn, (T *)h->tbuf, lo, sc);
     if (h->limType == DGADV_LIM_STRICT)
-      launch_k(h, k_limit<T, P, 2>, grid, SR::bytes(SR::lim(), 1), g, (const T *)h->tbuf, (T *)h->cn, lim_in<T>(lo, h), sc);
+      launch_k(h, k_limit<T, P, 2>, grid, SR::bytes(SR::lim(), 1) + vt_bytes<T>(h, 1), g, (const T *)h->tbuf, (T *)h->cn, lim_in<T>(lo, h), sc);
     else
-      launch_k(h, k_limit<T, P, 1>, grid, SR::bytes(SR::lim(), 1), g, (const T *)h->tbuf, (T *)h->cn, lim_in<T>(lo, h), sc);
+      launch_k(h, k_limit<T, P, 1>, grid, SR::bytes(SR::lim(), 1) + vt_bytes<T>(h, 1), g, (const T *)h->tbuf, (T *)h->cn, lim_in<T>(lo, h), sc);
   }
   return cudaGetLastError();
 }

@@ -93,7 +93,7 @@ __global__ void __launch_bounds__(kBlock) k_link_lim(const __grid_constant__ Lin
     if (q.p == 3) { limit_lin_tile<T, 3>(q.g, q.a, q.out, q.li, q.sc, tile); return; }
 }
 
-// Largest dynamic shared memory a linked stage kernel needs over the degrees of MASK.
+// Largest dynamic shared memory a linked stage kernel needs for its rows over the degrees of MASK.
 template <typename T, int MASK>
 static size_t link_smem(int kind) {
   size_t b = 0;
@@ -120,7 +120,9 @@ static cudaError_t launch_linked_step(dgadv_handle **hs, int n, double /*t0: no 
                                       double tau) {
   static_assert((MASK & 1) == 0, "linked steps cover degrees 1..3");
   dgadv_handle *h0 = hs[0];
-  const size_t smemOp = link_smem<T, MASK>(0), smemLd = link_smem<T, MASK>(1);
+  size_t vt = 0;                                        // the longest vertex table among the parts
+  for (int i = 0; i < n; ++i) vt = std::max(vt, vt_bytes<T>(hs[i], 1));
+  const size_t smemOp = link_smem<T, MASK>(0) + vt, smemLd = link_smem<T, MASK>(1) + 2 * vt, smemLm = vt;
   cudaError_t e = cudaFuncSetAttribute((const void *)k_link_op<T, MASK>,
                                        cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smemOp);
   if (e == cudaSuccess)
@@ -182,7 +184,7 @@ static cudaError_t launch_linked_step(dgadv_handle **hs, int n, double /*t0: no 
     }
     if (op.n) { prof_mark(h0, 0); launch_kb(h0, k_link_op<T, MASK>, gOp, eb, smemOp, op); prof_mark(h0, -1); }
     if (ld.n) { prof_mark(h0, 1); launch_k(h0, k_link_limdot<T, MASK>, gLd, smemLd, ld); prof_mark(h0, -1); }
-    if (lm.n) { prof_mark(h0, 2); launch_k(h0, k_link_lim<T, MASK>, gLm, (size_t)0, lm); prof_mark(h0, -1); }
+    if (lm.n) { prof_mark(h0, 2); launch_k(h0, k_link_lim<T, MASK>, gLm, smemLm, lm); prof_mark(h0, -1); }
   }
   for (int i = 0; i < n; ++i)
     if (S[i] == 1)                   // a one-stage step wrote cA (its input is c^n itself)

@@ -89,6 +89,10 @@ __device__ __forceinline__ void end_tile_barrier(const Geo<T> &g, int tile, int 
   }
 }
 
+// A tile's plain writes to shared memory (its vertex tables) before a later tile's bulk copies to the
+// same place; a block barrier follows.
+__device__ __forceinline__ void tile_fence() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
+
 // LIMMODE 0: no limiter; 1: linear limiter at p = 1; 2: linear limiter at p >= 2 (with the
 // time-derivative limiter).  Time-independent data without source terms.
 template <typename T, int P, int LIMMODE>
@@ -106,6 +110,7 @@ __global__ void __launch_bounds__(kBlock) k_step_persistent(const PersistArgs<T>
         if constexpr (std::is_same_v<T, double>)
           if (elem) stage_op_tile<T, P, 0, false, false, kOpElement>(a.g, in, a.cn, out, a.lo1[s], a.sc[s], tile);
         if (!elem) stage_op_tile<T, P, 0, false, false>(a.g, in, a.cn, out, a.lo1[s], a.sc[s], tile);
+        tile_fence();
         __syncthreads();
         end_tile_barrier<T, P>(a.g, tile, SR::op(0, false, elem));
       }
@@ -117,6 +122,7 @@ __global__ void __launch_bounds__(kBlock) k_step_persistent(const PersistArgs<T>
       if constexpr (std::is_same_v<T, double>)
         if (elem) stage_op_tile<T, P, (LIMMODE == 2 ? 2 : 1), false, true, kOpElement>(a.g, in, a.cn, a.tb, a.lo1[s], a.sc[s], tile);
       if (!elem) stage_op_tile<T, P, (LIMMODE == 2 ? 2 : 1), false, true>(a.g, in, a.cn, a.tb, a.lo1[s], a.sc[s], tile);
+      tile_fence();
       __syncthreads();
       end_tile_barrier<T, P>(a.g, tile, SR::op(LIMMODE == 2 ? 2 : 1, true, elem));
     }
@@ -125,6 +131,7 @@ __global__ void __launch_bounds__(kBlock) k_step_persistent(const PersistArgs<T>
       // time-derivative limiter, Taylor mass correction, SSP update, means scattered
       for (int tile = blockIdx.x; tile < a.nTiles; tile += gridDim.x) {
         limit_dot_lin_tile<T, P>(a.g, in, a.cn, a.tb, a.tb, a.li1[s], a.lo2[s], a.sc[s], tile);
+        tile_fence();
         __syncthreads();
         end_tile_barrier<T, P>(a.g, tile, SR::limdot_lin_rows(a.g.mtOnTheFly != 0));
       }
@@ -133,6 +140,7 @@ __global__ void __launch_bounds__(kBlock) k_step_persistent(const PersistArgs<T>
     // solution limiter
     for (int tile = blockIdx.x; tile < a.nTilesK; tile += gridDim.x) {
       limit_lin_tile<T, P>(a.g, a.tb, out, LIMMODE == 2 ? a.li2[s] : a.li1[s], a.scBC[s], tile);
+      tile_fence();
       __syncthreads();
     }
     if (!grid_sync(a.bar, a.sc[s].flag)) return;
@@ -152,7 +160,7 @@ static size_t persist_smem() {
   b = std::max(b, SR::bytes(SR::op(1, true, e), 1));
   b = std::max(b, SR::bytes(SR::op(2, true, e), 1));
   b = std::max(b, SR::bytes(SR::limdot_lin(), 1));
-  return b;
+  return b + vt_most<T, 1>(2);   // one quantity: the linear limiter
 }
 
 template <typename T, int P>

@@ -226,6 +226,23 @@ static int create_impl(const dgadv_mesh *mesh, const dgadv_params *prm, const st
     h->detJ[k] = gr.detJ0T[t];
     for (int i = 0; i < 4; ++i) { Bsoa[(size_t)i * Kp + k] = gr.B[4 * (size_t)t + i]; h->Bhost[4 * (size_t)k + i] = gr.B[4 * (size_t)t + i]; }
   }
+  // the vertices of each block of kBlock elements, and the elements' positions in their block's list
+  std::vector<int> vtPtr(1, 0), vtIdx;
+  std::vector<unsigned short> vtLoc(3 * (size_t)Kp, 0);
+  for (int b = 0; b < Kp; b += kBlock) {
+    std::vector<int> v;
+    for (int k = b; k < std::min(b + kBlock, K); ++k)
+      for (int n = 0; n < 3; ++n) v.push_back(V0T[(size_t)n * Kp + k]);
+    std::sort(v.begin(), v.end());
+    v.erase(std::unique(v.begin(), v.end()), v.end());
+    for (int k = b; k < std::min(b + kBlock, K); ++k)
+      for (int n = 0; n < 3; ++n)
+        vtLoc[(size_t)n * Kp + k] = (unsigned short)(std::lower_bound(v.begin(), v.end(), V0T[(size_t)n * Kp + k]) - v.begin());
+    vtIdx.insert(vtIdx.end(), v.begin(), v.end());
+    vtPtr.push_back((int)vtIdx.size());
+    h->vtMax = std::max(h->vtMax, (int)v.size());
+  }
+  if (!h->lim) h->vtMax = 0;   // the limiter's kernels alone use them
   // CSR vertex -> elements (internal ids)
   std::vector<int> vptr(h->numV + 1, 0), vidx(3 * (size_t)K);
   for (int k = 0; k < K; ++k)
@@ -292,6 +309,14 @@ static int create_impl(const dgadv_mesh *mesh, const dgadv_params *prm, const st
   if ((st = upload(h, h->vptr, vptr.data(), vptr.size() * 4))) return st;
   if ((st = upload(h, h->vidx, vidx.data(), vidx.size() * 4))) return st;
   if ((st = upload(h, h->perm, perm.data(), perm.size() * 4))) return st;
+  if (h->vtMax) {
+    if ((st = dev_alloc(h, (void **)&h->vtPtr, vtPtr.size() * 4))) return st;
+    if ((st = dev_alloc(h, (void **)&h->vtIdx, vtIdx.size() * 4))) return st;
+    if ((st = dev_alloc(h, (void **)&h->vtLoc, vtLoc.size() * 2))) return st;
+    if ((st = upload(h, h->vtPtr, vtPtr.data(), vtPtr.size() * 4))) return st;
+    if ((st = upload(h, h->vtIdx, vtIdx.data(), vtIdx.size() * 4))) return st;
+    if ((st = upload(h, h->vtLoc, vtLoc.data(), vtLoc.size() * 2))) return st;
+  }
   if (h->nInst > 1) {
     // instance of every block a kernel may launch (grids cover max(K, numV) elements)
     const int nBlocks = (std::max(Kp, h->Vp) + kBlock - 1) / kBlock + 1;
