@@ -210,13 +210,25 @@ struct LimVjpArgs {
                        // record set, pass mod adjKeySets); only lambda is applied here
 };
 
-// One stage of one transported species (dgadv_transport.cu): c h out from c h in, the
-// step's c h, the species' concentration and mask.
-struct TrStageArgs {
-  const void *conc, *cHin, *cH0;
-  void *cHout;
-  const uint8_t *mask;
+// One stage of every transported species (dgadv_transport.cu); arrays of all species, species s at
+// s times their size (N Kp reals, Kp mask bytes).
+struct TrArgs {
+  int nSpecies;
+  void *conc;             // limited concentrations
+  void *work;             // unlimited ones, between the two kernels of a stage
+  const void *cHin;       // c h before the stage (init: the projected initial data)
+  const void *cH0;        // c h at the start of the step
+  void *cHout;            // c h after the stage
+  uint8_t *mask;
+  const void *hQ;         // depth at the volume points, Q x Kp
+  void *vkeys;            // 3 passes x nSpecies x 2 x Vp
+  unsigned long long *slots;   // 3 passes x nSpecies x nInst x kSlotCopies x 2
+  long long pass;         // limiter passes so far
   double omega, tau;
+  double gco[4];          // time factors of the limiter's boundary data
+  bool init;              // initial data: no stage, c h taken from cHin
+  bool updateMask;        // this pass's patch extremes give the masks
+  double maskTol;
 };
 
 // Work of one arithmetic type, enqueued on the handle's stream.
@@ -257,9 +269,8 @@ struct PrecOps {
   // FP64: the digits of the linear limiter's correction rows (null: not used)
   cudaError_t (*fix_correction)(dgadv_handle *h);
   // transport problem (null: not built for this type)
-  cudaError_t (*tr_stage)(dgadv_handle *h, const TrStageArgs &a);
-  cudaError_t (*tr_convert)(dgadv_handle *h, const void *in, void *out, const void *hQ, int toConc);
-  cudaError_t (*tr_mask)(dgadv_handle *h, long long pass, double tol, uint8_t *mask);
+  cudaError_t (*tr_stage)(dgadv_handle *h, const TrArgs &a);   // cHin, conc -> work, means scattered
+  cudaError_t (*tr_limit)(dgadv_handle *h, const TrArgs &a);   // work -> conc, cHout, masks
 };
 
 // Fused path (linear limiter, zero Dirichlet data, opted in): per stage the operator kernel

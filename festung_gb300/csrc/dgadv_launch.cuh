@@ -721,8 +721,7 @@ static PrecOps make_ops() {
   o.fix_correction = nullptr;
   if constexpr (std::is_same_v<T, double>) o.fix_correction = dispatch_fix_correction<T>;
   o.tr_stage = nullptr;
-  o.tr_convert = nullptr;
-  o.tr_mask = nullptr;
+  o.tr_limit = nullptr;
   return o;
 }
 
