@@ -21,16 +21,21 @@
 #include <string>
 #include <vector>
 
+#include "dgadv_fixed.cuh"
 #include "dgadv_handle.h"
 
 namespace dgadv {
 namespace {
 
 constexpr int kImplBlock = 128;
-constexpr int kElemThreads = 32;      // element kernels: one warp per block spreads a small mesh over every SM
+// Every kernel over the elements runs blocks of 32 elements x N coefficient rows, a warp per row: FP64
+// instructions issue at their full (low) rate only with warps on all four schedulers of an SM, and
+// the reference's 8192 elements are 256 warps with a thread per element, under two per SM.
+constexpr int kRows = 32;             // elements per block
+constexpr int kVecs = 8;              // basis vectors a thread has in flight at once
+constexpr int kCheck = 4;             // Arnoldi steps between two looks at the residual estimate
 constexpr int kVecThreads = 256;
-constexpr int kMaxDotBlocks = 512;
-constexpr int kChunk = 8;             // vectors per multi-dot / update launch
+constexpr int kChunk = 8;             // vectors per linear combination launch
 
 template <int P> struct IDims {
   static constexpr int N = (P + 1) * (P + 2) / 2;
@@ -46,6 +51,7 @@ template <typename T, int P> struct ImplTab {
   T phi1D[3][R][N];
   T thetaPhi[3][3][R][N];
   T hatMinv[N][N];
+  T Fphi[3][R][N];    // hatM^-1 applied to the edge test functions
 };
 
 __constant__ ImplTab<double, 0> c_d0;
@@ -81,76 +87,100 @@ template <typename T> struct ImplArgs {
   int K, Kp, nTerms;
   const T *F, *Vn, *rhs;
   const int *nbr, *code;
+  const T *A;          // N^2 x Kp: cDot's local part (volume term and own outflow, mass solve applied)
   double gco[4];       // g_m(t) of the source terms
 };
 
-// y = ca x + cb cDot(x), cDot = M^-1 (sum_m g_m rhs_m [RHS] + volume(x) - upwind flux(x)).
-template <typename T, int P, bool RHS>
-__global__ void __launch_bounds__(kImplBlock) k_impl_op(const ImplArgs<T> a, const T *__restrict__ x,
-                                                        T *__restrict__ y, double ca, double cb) {
-  constexpr int N = IDims<P>::N, Q = IDims<P>::Q, R = IDims<P>::R;
-  const int k = blockIdx.x * blockDim.x + threadIdx.x;
-  if (k >= a.K) return;
+// Coefficient `row` of cDot(x)'s parts for element k, by the block's N warps together (row = the warp,
+// element = the lane):
+//   LOCAL: the local part, the row of the element's matrix (volume term and own outflow, hatM^-1
+//          applied), 6 multiply-adds at p = 2 and 10 at p = 3 where the quadrature form of the whole
+//          element has 180 and 1600;
+//   minus the inflow terms, the part that couples elements: the warps share the 3 R edge points
+//          (trace of the neighbour times the velocity, into fl), then every row adds its test functions.
+// Contains a block barrier.
+template <typename T, int P> struct EdgePoints {   // a warp's edge points, all loads in flight together
+  static constexpr int M = (3 * IDims<P>::R + IDims<P>::N - 1) / IDims<P>::N;
+  int code, nb[M];
+  T v[M];
+  __device__ __forceinline__ void load(const ImplArgs<T> &a, int k, bool act) {
+    code = act ? a.code[k] : 0;
+#pragma unroll
+    for (int i = 0; i < M; ++i) {
+      const int pt = threadIdx.y + i * IDims<P>::N;
+      const bool use = act && pt < 3 * IDims<P>::R;
+      nb[i] = use ? a.nbr[(size_t)(pt / IDims<P>::R) * a.Kp + k] : -1;
+      v[i] = use ? a.Vn[(size_t)pt * a.Kp + k] : T(0);
+    }
+  }
+};
+template <typename T, int P, bool LOCAL>
+__device__ __forceinline__ T cdot_row(const ImplArgs<T> &a, const EdgePoints<T, P> &ep, const T *x, int k, bool act,
+                                      T (*fl)[kRows]) {
+  constexpr int N = IDims<P>::N, R = IDims<P>::R;
   const ImplTab<T, P> &tb = itab<T, P>();
   const size_t Kp = a.Kp;
-  T c[N], rhs[N];
+  const int lane = threadIdx.x, row = threadIdx.y;
 #pragma unroll
-  for (int i = 0; i < N; ++i) { c[i] = x[i * Kp + k]; rhs[i] = T(0); }
+  for (int i = 0; i < EdgePoints<T, P>::M; ++i) {
+    const int pt = row + i * N;
+    if (pt >= 3 * R) break;
+    const int n = pt / R, r = pt - n * R;
+    T f = T(0);
+    if (ep.v[i] < T(0) && ep.nb[i] >= 0) {
+      const T *th = tb.thetaPhi[n][(ep.code >> (2 * n)) & 3][r];
+      T tr = T(0);
+#pragma unroll
+      for (int j = 0; j < N; ++j) tr = fma(th[j], x[j * Kp + ep.nb[i]], tr);
+      f = ep.v[i] * tr;
+    }
+    fl[pt][lane] = f;
+  }
+  T s = T(0);
+  if (LOCAL && act) {
+#pragma unroll
+    for (int j = 0; j < N; ++j) s = fma(a.A[(size_t)(row * N + j) * Kp + k], x[j * Kp + k], s);
+  }
+  __syncthreads();
+#pragma unroll
+  for (int n = 0; n < 3; ++n)
+#pragma unroll
+    for (int r = 0; r < R; ++r) s = fma(-tb.Fphi[n][r][row], fl[n * R + r][lane], s);
+  return s;
+}
+
+// y = ca x + cb cDot(x), cDot with the source terms M^-1 sum_m g_m rhs_m [RHS].
+template <typename T, int P, bool RHS>
+__global__ void __launch_bounds__(kRows * IDims<P>::N) k_impl_op(const ImplArgs<T> a, const T *__restrict__ x,
+                                                                 T *__restrict__ y, double ca, double cb) {
+  constexpr int N = IDims<P>::N;
+  __shared__ T fl[3 * IDims<P>::R][kRows];
+  const int k = blockIdx.x * kRows + threadIdx.x, row = threadIdx.y;
+  const size_t Kp = a.Kp;
+  const bool act = k < a.K;
+  EdgePoints<T, P> ep;
+  ep.load(a, k, act);
+  T s = cdot_row<T, P, true>(a, ep, x, k, act, fl);
+  if (!act) return;
   if (RHS) {
     for (int m = 0; m < a.nTerms; ++m) {
-      const T gm = T(a.gco[m]);
+      T q = T(0);
 #pragma unroll
-      for (int i = 0; i < N; ++i) rhs[i] = fma(gm, a.rhs[(m * N + i) * Kp + k], rhs[i]);
+      for (int j = 0; j < N; ++j) q = fma(itab<T, P>().hatMinv[row][j], a.rhs[(size_t)(m * N + j) * Kp + k], q);
+      s = fma(T(a.gco[m]), q, s);
     }
   }
-#pragma unroll 1
-  for (int q = 0; q < Q; ++q) {
-    T cq = T(0);
-#pragma unroll
-    for (int j = 0; j < N; ++j) cq = fma(tb.phiQ[q][j], c[j], cq);
-    const T f1 = a.F[q * Kp + k] * cq, f2 = a.F[(Q + q) * Kp + k] * cq;
-#pragma unroll
-    for (int i = 0; i < N; ++i) rhs[i] = fma(tb.g2[q][i], f2, fma(tb.g1[q][i], f1, rhs[i]));
-  }
-  const int code = a.code[k];
-#pragma unroll
-  for (int n = 0; n < 3; ++n) {
-    const int nb = a.nbr[n * Kp + k];
-    const int np = (code >> (2 * n)) & 3;
-    const bool outOk = (code >> (6 + n)) & 1;
-    T cn[N];
-#pragma unroll
-    for (int j = 0; j < N; ++j) cn[j] = nb >= 0 ? x[j * Kp + nb] : T(0);
-#pragma unroll
-    for (int r = 0; r < R; ++r) {
-      const T v = a.Vn[(n * R + r) * Kp + k];
-      T tr = T(0);
-      if (v > T(0) && outOk) {
-#pragma unroll
-        for (int j = 0; j < N; ++j) tr = fma(tb.phi1D[n][r][j], c[j], tr);
-      } else if (v < T(0) && nb >= 0) {
-        for (int j = 0; j < N; ++j) tr = fma(tb.thetaPhi[n][np & 3][r][j], cn[j], tr);
-      }
-      const T fl = v * tr;
-#pragma unroll
-      for (int i = 0; i < N; ++i) rhs[i] = fma(-tb.phi1D[n][r][i], fl, rhs[i]);
-    }
-  }
-#pragma unroll
-  for (int i = 0; i < N; ++i) {
-    T s = T(0);
-#pragma unroll
-    for (int j = 0; j < N; ++j) s = fma(tb.hatMinv[i][j], rhs[j], s);
-    y[i * Kp + k] = T(ca) * c[i] + T(cb) * s;
-  }
+  y[row * Kp + k] = T(ca) * x[row * Kp + k] + T(cb) * s;
 }
 
 // Inverse of each element's diagonal block of y = ca x + cb cDot(x) (volume term and the
 // element's own outflow; the neighbours' inflow is off-diagonal), by Gauss-Jordan elimination
-// with partial pivoting in FP64.  A block with a vanishing pivot is replaced by the identity.
+// with partial pivoting in FP64.  A block with a vanishing pivot is replaced by the identity and
+// *singular set.  Aloc receives cDot's local part itself.
 template <typename T, int P>
 __global__ void __launch_bounds__(kImplBlock) k_impl_block(const ImplArgs<T> a, double ca, double cb,
-                                                           T *__restrict__ Pinv) {
+                                                           T *__restrict__ Pinv, T *__restrict__ Aloc,
+                                                           int *__restrict__ singular) {
   constexpr int N = IDims<P>::N, Q = IDims<P>::Q, R = IDims<P>::R;
   const int k = blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= a.K) return;
@@ -187,6 +217,7 @@ __global__ void __launch_bounds__(kImplBlock) k_impl_block(const ImplArgs<T> a, 
     for (int j = 0; j < N; ++j) {
       double s = 0.0;
       for (int l = 0; l < N; ++l) s += (double)tb.hatMinv[i][l] * J[l][j];
+      Aloc[(size_t)(i * N + j) * Kp + k] = T(s);
       A[i][j] = (i == j ? ca : 0.0) + cb * s;
       A[i][N + j] = i == j ? 1.0 : 0.0;
     }
@@ -208,51 +239,132 @@ __global__ void __launch_bounds__(kImplBlock) k_impl_block(const ImplArgs<T> a, 
         for (int j = 0; j < 2 * N; ++j) A[r][j] -= f * A[col][j];
     }
   }
+  if (!ok) *singular = 1;
   for (int i = 0; i < N; ++i)
     for (int j = 0; j < N; ++j) Pinv[(i * N + j) * Kp + k] = T(ok ? A[i][N + j] : (i == j ? 1.0 : 0.0));
 }
 
-template <typename T, int P>
-__global__ void __launch_bounds__(kImplBlock) k_impl_prec(int K, int Kp, const T *__restrict__ Pinv,
-                                                          const T *__restrict__ r, T *__restrict__ z) {
-  constexpr int N = IDims<P>::N;
-  const int k = blockIdx.x * blockDim.x + threadIdx.x;
-  if (k >= K) return;
-  T rv[N];
-#pragma unroll
-  for (int j = 0; j < N; ++j) rv[j] = r[(size_t)j * Kp + k];
-#pragma unroll
-  for (int i = 0; i < N; ++i) {
-    T s = T(0);
-#pragma unroll
-    for (int j = 0; j < N; ++j) s = fma(Pinv[(size_t)(i * N + j) * Kp + k], rv[j], s);
-    z[(size_t)i * Kp + k] = s;
-  }
-}
-
 // ---- vector kernels over n = N Kp values ------------------------------------------------------
 
-__device__ __forceinline__ double block_sum(double v, double *sh) {
+// A sum over the grid in a fixed order: every block adds its threads' shares, the block that
+// arrives last adds the blocks' (in block order, whichever block it is).
+struct GridSums {
+  double *partial;          // vector v, block b at v * gridDim.x + b
+  unsigned int *ticket;     // blocks that have stored their shares (0 between launches)
+  double *out;
+};
+// Sums x[0 .. n) over a warp's lanes, in every lane.  On the integer units: each share scaled to 57 bits
+// below the lanes' largest exponent (off by at most 2^-57 of it, where an FP64 addition rounds at
+// 2^-53), one redux and five exchanges and additions of 64-bit words, n sums side by side; five FP64
+// additions each would hold the warp's scheduler for 380 cycles.  Shares outside 2^(+-800) take the
+// FP64 form.
+template <int n> __device__ __forceinline__ void warp_sums(double x[n]) {
+  int E[n];
+  bool ok = true;
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
-  const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
-  if (l == 0) sh[w] = v;
-  __syncthreads();
-  double s = 0.0;
-  if (threadIdx.x == 0)
-    for (int i = 0; i < (int)(blockDim.x >> 5); ++i) s += sh[i];
-  __syncthreads();
-  return s;
+  for (int q = 0; q < n; ++q) {
+    E[q] = __reduce_max_sync(0xffffffffu, __double2hiint(x[q]) & 0x7fffffff) >> 20;
+    ok = ok && (E[q] == 0 || (E[q] >= 223 && E[q] <= 1823));
+  }
+  if (!ok) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+      for (int q = 0; q < n; ++q) x[q] += __shfl_xor_sync(0xffffffffu, x[q], o);
+    return;
+  }
+  long long v[n];
+#pragma unroll
+  for (int q = 0; q < n; ++q) v[q] = fx::fix<57>(x[q], max(E[q], 223));   // all zero: zero
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+    for (int q = 0; q < n; ++q) v[q] += __shfl_xor_sync(0xffffffffu, v[q], o);
+#pragma unroll
+  for (int q = 0; q < n; ++q) x[q] = fx::to_double_int(v[q], max(E[q], 223) - 1022 - 57);
 }
-
-// out[v] = sum of nb partials of vector v (one block per vector, fixed order)
-__global__ void __launch_bounds__(kVecThreads) k_dot_final(const double *__restrict__ partial, int nb,
-                                                           double *__restrict__ out) {
-  __shared__ double sh[kVecThreads / 32];
-  double s = 0.0;
-  for (int i = threadIdx.x; i < nb; i += blockDim.x) s += partial[blockIdx.x * nb + i];
-  s = block_sum(s, sh);
-  if (threadIdx.x == 0) out[blockIdx.x] = s;
+// The threads' shares x[0 .. n) of vectors v0 ...: added over the block into partial.
+template <int N>
+__device__ __forceinline__ void store_shares(const GridSums &gs, int v0, int n, double x[kVecs]) {
+  __shared__ double sh[N][kVecs];
+  __syncthreads();                            // the shares before are read
+  if (n <= 2) warp_sums<2>(x);                // the values beyond n are zero
+  else if (n <= 4) warp_sums<4>(x);
+  else warp_sums<kVecs>(x);
+  if (threadIdx.x == 0)
+#pragma unroll
+    for (int q = 0; q < kVecs; ++q) sh[threadIdx.y][q] = x[q];
+  __syncthreads();
+  if (threadIdx.y == 0 && (int)threadIdx.x < n) {
+    double s = 0.0;
+#pragma unroll
+    for (int i = 0; i < N; ++i) s += sh[i][threadIdx.x];
+    gs.partial[(size_t)(v0 + threadIdx.x) * gridDim.x + blockIdx.x] = s;
+  }
+}
+// After the shares of nv vectors: the last block writes their sums.
+template <int N>
+__device__ __forceinline__ void finish_sums(const GridSums &gs, int nv) {
+  __shared__ bool last;
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0 && threadIdx.y == 0) last = atomicAdd(gs.ticket, 1u) == gridDim.x - 1;
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+  constexpr int kV = 2;                       // vectors of a warp at once
+  for (int v0 = kV * threadIdx.y; v0 < nv; v0 += kV * N) {
+    double s[kV] = {0.0, 0.0};
+#pragma unroll 8
+    for (int b = threadIdx.x; b < (int)gridDim.x; b += 32)
+#pragma unroll
+      for (int q = 0; q < kV; ++q)
+        if (v0 + q < nv) s[q] += __ldcg(&gs.partial[(size_t)(v0 + q) * gridDim.x + b]);
+    warp_sums<kV>(s);
+    if (threadIdx.x == 0)
+#pragma unroll
+      for (int q = 0; q < kV; ++q)
+        if (v0 + q < nv) gs.out[v0 + q] = s[q];
+  }
+  if (threadIdx.x == 0 && threadIdx.y == 0) *gs.ticket = 0;
+}
+// The shares of <V_v, y> for v < nv, at = row Kp + k the thread's place (inactive: y = 0, at within V).
+template <typename T, int N>
+__device__ __forceinline__ void share_products(const GridSums &gs, const T *V, size_t n, size_t at, int nv, double y) {
+  for (int v0 = 0; v0 < nv; v0 += kVecs) {
+    double s[kVecs];
+#pragma unroll
+    for (int q = 0; q < kVecs; ++q) s[q] = v0 + q < nv ? (double)V[(size_t)(v0 + q) * n + at] : 0.0;
+#pragma unroll
+    for (int q = 0; q < kVecs; ++q) s[q] *= y;
+    store_shares<N>(gs, v0, min(kVecs, nv - v0), s);
+  }
+}
+// y + sgn sum_{v < nv} h_v V_v at the thread's place
+template <typename T>
+__device__ __forceinline__ double add_vectors(const T *V, size_t n, size_t at, int nv, const double *h, double sgn,
+                                              double y) {
+  for (int v0 = 0; v0 < nv; v0 += kVecs) {
+    double a[kVecs];
+#pragma unroll
+    for (int q = 0; q < kVecs; ++q) a[q] = v0 + q < nv ? (double)V[(size_t)(v0 + q) * n + at] : 0.0;
+#pragma unroll
+    for (int q = 0; q < kVecs; ++q)
+      if (v0 + q < nv) y += sgn * h[v0 + q] * a[q];
+  }
+  return y;
+}
+// Row `row` of P^-1 v for the block's elements, v given a value per thread.  Contains a block barrier.
+template <typename T, int N>
+__device__ __forceinline__ T precondition_row(const T *Pinv, size_t Kp, int k, bool act, T v, T (*vs)[kRows]) {
+  vs[threadIdx.y][threadIdx.x] = v;
+  __syncthreads();
+  T s = T(0);
+  if (act) {
+#pragma unroll
+    for (int j = 0; j < N; ++j) s = fma(Pinv[(size_t)(threadIdx.y * N + j) * Kp + k], vs[j][threadIdx.x], s);
+  }
+  return s;
 }
 
 // y = sum_v c_v x_v (host coefficients, up to kChunk vectors; y may alias an input)
@@ -272,96 +384,234 @@ __global__ void __launch_bounds__(kVecThreads) k_comb(T *y, const Comb<T> cb, si
   }
 }
 
-// v = w / sqrt(nrm2[0]) (zero if the norm vanishes)
-template <typename T>
-__global__ void __launch_bounds__(kVecThreads) k_unit(T *__restrict__ v, const T *__restrict__ w,
-                                                      const double *__restrict__ nrm2, size_t n) {
-  const double s = nrm2[0] > 0.0 ? 1.0 / sqrt(nrm2[0]) : 0.0;
-  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x)
-    v[i] = T((double)w[i] * s);
-}
-
-// partial[v * gridDim.x + b] = block b's share of <V_v, w> for every v < nv, kChunk vectors per
-// pass over w
-template <typename T>
-__global__ void __launch_bounds__(kVecThreads) k_mdot_n(const T *__restrict__ V, size_t ldv, int nv,
-                                                        const T *__restrict__ w, size_t n, double *__restrict__ partial) {
-  __shared__ double sh[kVecThreads / 32];
-  for (int v0 = 0; v0 < nv; v0 += kChunk) {
-    const int c = min(kChunk, nv - v0);
-    double acc[kChunk];
-#pragma unroll
-    for (int v = 0; v < kChunk; ++v) acc[v] = 0.0;
-    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
-      const double wi = (double)w[i];
-#pragma unroll
-      for (int v = 0; v < kChunk; ++v)
-        if (v < c) acc[v] += (double)V[(size_t)(v0 + v) * ldv + i] * wi;
-    }
-    for (int v = 0; v < c; ++v) {
-      const double s = block_sum(acc[v], sh);
-      if (threadIdx.x == 0) partial[(size_t)(v0 + v) * gridDim.x + blockIdx.x] = s;
-    }
-  }
-}
-
-// y = ay y + sgn sum_{v < nv} coef[v] V_v (coefficients in device memory)
-template <typename T>
-__global__ void __launch_bounds__(kVecThreads) k_vcomb_n(T *__restrict__ y, double ay, const T *__restrict__ V,
-                                                         size_t ldv, int nv, const double *__restrict__ coef,
-                                                         double sgn, size_t n) {
-  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
-    double s = ay == 0.0 ? 0.0 : ay * (double)y[i];
-    for (int v = 0; v < nv; ++v) s += sgn * coef[v] * (double)V[(size_t)v * ldv + i];
-    y[i] = T(s);
-  }
-}
-
-// The small dense part of GMRES, one thread: Hessenberg column j from the two Gram-Schmidt
-// passes and |w|^2, the earlier Givens rotations, a new one, and the residual estimate.
+// The small dense part of GMRES: Hessenberg matrix, Givens rotations, residual estimate.
 // status: [0] |g_{j+1}|, [1] columns in use, [2] breakdown seen (later columns are ignored).
 struct GmresDense {
   double *H, *cs, *sn, *g, *y, *status;   // H: (m + 1) x m, column-major
 };
-__global__ void k_gmres_start(GmresDense d, const double *__restrict__ nrm2, int m) {
-  d.g[0] = sqrt(fmax(nrm2[0], 0.0));
-  for (int i = 1; i <= m; ++i) d.g[i] = 0.0;
-  d.status[0] = d.g[0];
-  d.status[1] = 0.0;
-  d.status[2] = 0.0;
-}
-__global__ void k_gmres_column(GmresDense d, const double *__restrict__ h1, const double *__restrict__ h2,
-                               const double *__restrict__ nrm2, int j, int m) {
-  if (d.status[2] != 0.0) return;
-  double *col = d.H + (size_t)j * (m + 1);
-  for (int i = 0; i <= j; ++i) col[i] = h1[i] + h2[i];
-  col[j + 1] = sqrt(fmax(nrm2[0], 0.0));
-  for (int i = 0; i < j; ++i) {
-    const double t0 = d.cs[i] * col[i] + d.sn[i] * col[i + 1];
-    col[i + 1] = -d.sn[i] * col[i] + d.cs[i] * col[i + 1];
-    col[i] = t0;
+
+// One Arnoldi step is three kernels over the elements (it was eleven launches and 90 us at 8192
+// elements, p = 2; now 45 us):
+//   k_arn_apply   w = A P^-1 v_j; h1 = V^T w.  z = P^-1 v_j comes from the step before.  P inverts the
+//                 element's own block of A, so the local part of A z is v_j itself and only the
+//                 neighbours' inflow is left (IDENT; a mesh with a singular block, whose P is the
+//                 identity there, applies the whole operator)
+//   k_arn_first   w -= V h1; h2 = V^T w and |w|^2        (classical Gram-Schmidt, second pass)
+//   k_arn_second  w -= V h2; v_{j+1} = w / |w|, with |w|^2 after the pass from |w|^2 - |h2|^2 (h2 is at
+//                 rounding level: no cancellation); z = P^-1 v_{j+1}; column j of the Hessenberg matrix and
+//                 the Givens rotations in one more block
+template <typename T, int P, bool IDENT>
+__global__ void __launch_bounds__(kRows * IDims<P>::N)
+k_arn_apply(const ImplArgs<T> a, const T *__restrict__ V, size_t n, int j, const T *__restrict__ z, T *__restrict__ w,
+            double ca, double cb, const GridSums gs) {
+  constexpr int N = IDims<P>::N;
+  __shared__ T fl[3 * IDims<P>::R][kRows];
+  const int k = blockIdx.x * kRows + threadIdx.x;
+  const bool act = k < a.K;
+  const size_t at = (size_t)threadIdx.y * a.Kp + (act ? k : 0);
+  EdgePoints<T, P> ep;
+  ep.load(a, k, act);
+  const T s = cdot_row<T, P, !IDENT>(a, ep, z, k, act, fl);
+  T y = T(0);
+  if (act) {
+    y = (IDENT ? V[(size_t)j * n + at] : T(ca) * z[at]) + T(cb) * s;
+    w[at] = y;
   }
-  const double r = hypot(col[j], col[j + 1]);
-  d.cs[j] = r > 0.0 ? col[j] / r : 1.0;
-  d.sn[j] = r > 0.0 ? col[j + 1] / r : 0.0;
-  col[j] = r;
-  col[j + 1] = 0.0;
-  d.g[j + 1] = -d.sn[j] * d.g[j];
-  d.g[j] = d.cs[j] * d.g[j];
-  d.status[0] = fabs(d.g[j + 1]);
-  d.status[1] = (double)(j + 1);
-  if (r == 0.0) d.status[2] = 1.0;
+  share_products<T, N>(gs, V, n, at, j + 1, (double)y);
+  finish_sums<N>(gs, j + 1);
 }
-// y = H^-1 g over the columns in use (upper triangular), zero beyond them.
+
+template <typename T, int N>
+__global__ void __launch_bounds__(kRows * N) k_arn_first(int K, int Kp, const T *V, size_t n, int j, T *w,
+                                                         const double *h1, const GridSums gs) {
+  __shared__ double sh[257];
+  for (int v = threadIdx.y * 32 + threadIdx.x; v <= j; v += 32 * N) sh[v] = h1[v];
+  const int k = blockIdx.x * kRows + threadIdx.x;
+  const bool act = k < K;
+  const size_t at = (size_t)threadIdx.y * Kp + (act ? k : 0);
+  double y = act ? (double)w[at] : 0.0;
+  __syncthreads();
+  if (act) {
+    const T t = T(add_vectors(V, n, at, j + 1, sh, -1.0, y));
+    w[at] = t;
+    y = (double)t;
+  }
+  share_products<T, N>(gs, V, n, at, j + 1, y);
+  double s[kVecs] = {y * y};
+  store_shares<N>(gs, j + 1, 1, s);
+  finish_sums<N>(gs, j + 2);
+}
+
+// Column j: h1 + h2, the earlier rotations, a new one, the residual estimate.  One warp; the chain of
+// rotations runs on one lane from shared memory.
+__device__ __forceinline__ void gmres_column(const GmresDense &d, const double *h1, const double *h2, double nrm2, int j,
+                                             int m, double *col, double *cs, double *sn) {
+  const int l = threadIdx.x;
+  for (int i = l; i <= j; i += 32) {
+    col[i] = h1[i] + h2[i];
+    if (i < j) { cs[i] = d.cs[i]; sn[i] = d.sn[i]; }
+  }
+  __syncwarp();
+  if (l == 0 && d.status[2] == 0.0) {
+    double c0 = col[0];
+    for (int i = 0; i < j; ++i) {
+      const double c1 = col[i + 1];
+      col[i] = cs[i] * c0 + sn[i] * c1;
+      c0 = -sn[i] * c0 + cs[i] * c1;
+    }
+    const double nw = sqrt(fmax(nrm2, 0.0));
+    const double r = hypot(c0, nw);
+    const double c = r > 0.0 ? c0 / r : 1.0, s = r > 0.0 ? nw / r : 0.0;
+    d.cs[j] = c;
+    d.sn[j] = s;
+    col[j] = r;
+    const double g = d.g[j];
+    d.g[j + 1] = -s * g;
+    d.g[j] = c * g;
+    d.status[0] = fabs(s * g);
+    d.status[1] = (double)(j + 1);
+    if (r == 0.0) d.status[2] = 1.0;
+    cs[0] = 1.0;   // the column counts
+  } else if (l == 0) {
+    cs[0] = 0.0;
+  }
+  __syncwarp();
+  if (cs[0] != 0.0)
+    for (int i = l; i <= j; i += 32) d.H[(size_t)j * (m + 1) + i] = col[i];
+  if (l == 0 && cs[0] != 0.0) d.H[(size_t)j * (m + 1) + j + 1] = 0.0;
+}
+
+// h2: then |w|^2 at j + 1.  The last block has no elements: the column.
+template <typename T, int N>
+__global__ void __launch_bounds__(kRows * N)
+k_arn_second(int K, int Kp, T *V, size_t n, int j, const T *w, const T *__restrict__ Pinv, T *z, const double *h1,
+             const double *h2, GmresDense d, int m) {
+  __shared__ double col[257], cs[257], sn[257];
+  __shared__ double norm;
+  __shared__ T vs[N][kRows];
+  const int k = blockIdx.x * kRows + threadIdx.x;
+  const bool act = blockIdx.x != gridDim.x - 1 && k < K;
+  T pr[N];                  // the row of P^-1, in flight with the rest
+#pragma unroll
+  for (int i = 0; i < N; ++i) pr[i] = act ? Pinv[(size_t)(threadIdx.y * N + i) * Kp + k] : T(0);
+  if (threadIdx.y == 0) {   // |w|^2 - |h2|^2
+    double q[1] = {0.0};
+    for (int v = threadIdx.x; v <= j; v += 32) {
+      col[v] = h2[v];
+      q[0] += col[v] * col[v];
+    }
+    warp_sums<1>(q);
+    if (threadIdx.x == 0) norm = h2[j + 1] - q[0];
+  }
+  const size_t at = (size_t)threadIdx.y * Kp + (act ? k : 0);
+  double y = act ? (double)w[at] : 0.0;
+  __syncthreads();
+  const double nrm2 = norm;
+  if (blockIdx.x == gridDim.x - 1) {
+    if (threadIdx.y == 0) gmres_column(d, h1, h2, nrm2, j, m, col, cs, sn);
+    return;
+  }
+  const double s = nrm2 > 0.0 ? 1.0 / sqrt(nrm2) : 0.0;
+  T v1 = T(0);
+  if (act) {
+    v1 = T(add_vectors(V, n, at, j + 1, col, -1.0, y) * s);
+    V[(size_t)(j + 1) * n + at] = v1;
+  }
+  vs[threadIdx.y][threadIdx.x] = v1;
+  __syncthreads();
+  T zz = T(0);
+#pragma unroll
+  for (int i = 0; i < N; ++i) zz = fma(pr[i], vs[i][threadIdx.x], zz);
+  if (act) z[at] = zz;
+}
+
+// r = b - (ca x + cb cDot(x)), gs.out[0] = |r|^2, [1] = |b|^2
+template <typename T, int P>
+__global__ void __launch_bounds__(kRows * IDims<P>::N)
+k_impl_residual(const ImplArgs<T> a, const T *__restrict__ b, const T *__restrict__ x, T *__restrict__ r, double ca,
+                double cb, const GridSums gs) {
+  constexpr int N = IDims<P>::N;
+  __shared__ T fl[3 * IDims<P>::R][kRows];
+  const int k = blockIdx.x * kRows + threadIdx.x;
+  const bool act = k < a.K;
+  const size_t at = (size_t)threadIdx.y * a.Kp + (act ? k : 0);
+  EdgePoints<T, P> ep;
+  ep.load(a, k, act);
+  const T s = cdot_row<T, P, true>(a, ep, x, k, act, fl);
+  double q[kVecs] = {0.0};
+  if (act) {
+    const T bi = b[at], y = T(ca) * x[at] + T(cb) * s, ri = T((double)bi - (double)y);
+    r[at] = ri;
+    q[0] = (double)ri * (double)ri;
+    q[1] = (double)bi * (double)bi;
+  }
+  store_shares<N>(gs, 0, 2, q);
+  finish_sums<N>(gs, 2);
+}
+
+// v_0 = r / |r|, z = P^-1 v_0, and the dense part of a new cycle.
+template <typename T, int N>
+__global__ void __launch_bounds__(kRows * N) k_arn_start(int K, int Kp, const T *__restrict__ r, T *__restrict__ V,
+                                                         const T *__restrict__ Pinv, T *__restrict__ z,
+                                                         const double *__restrict__ nrm2, GmresDense d, int m) {
+  __shared__ T vs[N][kRows];
+  const int k = blockIdx.x * kRows + threadIdx.x;
+  const bool act = k < K;
+  const size_t at = (size_t)threadIdx.y * Kp + (act ? k : 0);
+  const double nr = nrm2[0];
+  if (blockIdx.x == 0 && threadIdx.y == 0) {
+    for (int i = threadIdx.x; i <= m; i += 32) d.g[i] = i == 0 ? sqrt(fmax(nr, 0.0)) : 0.0;
+    if (threadIdx.x == 0) { d.status[0] = sqrt(fmax(nr, 0.0)); d.status[1] = 0.0; d.status[2] = 0.0; }
+  }
+  T v = T(0);
+  if (act) {
+    v = T((double)r[at] * (nr > 0.0 ? 1.0 / sqrt(nr) : 0.0));
+    V[at] = v;
+  }
+  const T zz = precondition_row<T, N>(Pinv, Kp, k, act, v, vs);
+  if (act) z[at] = zz;
+}
+
+// y = H^-1 g over the columns in use (upper triangular), zero beyond them.  The columns come to shared
+// memory first (up to kSolveCols of them); then one warp takes each solved unknown off the rows
+// above it, the lanes side by side.
+constexpr int kSolveCols = 64;
 __global__ void k_gmres_solve(GmresDense d, int m) {
-  const int je = (int)d.status[1];
-  for (int i = m - 1; i >= je; --i) d.y[i] = 0.0;
-  for (int i = je - 1; i >= 0; --i) {
-    double s = d.g[i];
-    for (int l = i + 1; l < je; ++l) s -= d.H[(size_t)l * (m + 1) + i] * d.y[l];
-    const double diag = d.H[(size_t)i * (m + 1) + i];
-    d.y[i] = diag != 0.0 ? s / diag : 0.0;
+  __shared__ double g[256], H[kSolveCols * (kSolveCols + 1)];
+  const int je = (int)d.status[1], l = threadIdx.x;
+  const bool held = je <= kSolveCols;
+  for (int i = l; i < m; i += blockDim.x) {
+    if (i < je) g[i] = d.g[i];
+    else d.y[i] = 0.0;
   }
+  if (held)
+    for (int e = l; e < je * je; e += blockDim.x) {
+      const int c = e / je, r = e - c * je;
+      H[c * (kSolveCols + 1) + r] = d.H[(size_t)c * (m + 1) + r];
+    }
+  __syncthreads();
+  if (l >= 32) return;
+  for (int i = je - 1; i >= 0; --i) {
+    const double *col = held ? &H[i * (kSolveCols + 1)] : &d.H[(size_t)i * (m + 1)];
+    const double y = col[i] != 0.0 ? g[i] / col[i] : 0.0;
+    for (int q = l; q < i; q += 32) g[q] -= col[q] * y;
+    if (l == 0) d.y[i] = y;
+    __syncwarp();
+  }
+}
+
+// x += P^-1 V y over nv vectors
+template <typename T, int N>
+__global__ void __launch_bounds__(kRows * N) k_arn_update(int K, int Kp, const T *__restrict__ V, size_t n, int nv,
+                                                          const double *__restrict__ y, const T *__restrict__ Pinv,
+                                                          T *__restrict__ x) {
+  __shared__ T vs[N][kRows];
+  const int k = blockIdx.x * kRows + threadIdx.x;
+  const bool act = k < K;
+  const size_t at = (size_t)threadIdx.y * Kp + (act ? k : 0);
+  const T t = act ? T(add_vectors(V, n, at, nv, y, 1.0, 0.0)) : T(0);
+  const T z = precondition_row<T, N>(Pinv, Kp, k, act, t, vs);
+  if (act) x[at] = T((double)x[at] + (double)z);
 }
 
 double time_factor_of(int fn, double t) { return fn == DGADV_TIME_EXP_NEG ? std::exp(-t) : 1.0; }
@@ -412,9 +662,13 @@ struct ImplicitState {
   void *Pinv = nullptr;           // N^2 x Kp
   double pinvA = 0.0, pinvB = 0.0;
   int pinvVersion = -1;           // velocity version the blocks were built for
-  double *partial = nullptr;      // kChunk x kMaxDotBlocks
-  double *dres = nullptr;         // 3 x (m + 2): h1, h2, |w|^2
-  double *dcoef = nullptr;        // m + 1 coefficients
+  void *Aloc = nullptr;           // N^2 x Kp: cDot's local part
+  int *singular = nullptr;        // a diagonal block was singular
+  bool ident = false;             // ... none was: P^-1 inverts every diagonal block
+  int blocks = 0;                 // the element kernels' blocks
+  double *partial = nullptr;      // (m + 2) x blocks
+  unsigned int *ticket = nullptr;
+  double *dres = nullptr;         // h1 (m + 1), h2 and |w|^2 (m + 2)
   double *dense = nullptr;        // H ((m + 1) x m), cs, sn, g, y, status
   std::vector<cudaGraphExec_t> arnoldi;   // Arnoldi step j as a CUDA graph, for (graphA, graphB)
   double graphA = 0.0, graphB = 0.0;
@@ -454,6 +708,13 @@ cudaError_t upload_itab(const RefTables &rt, cudaStream_t stream) {
       }
   for (int i = 0; i < I::N; ++i)
     for (int j = 0; j < I::N; ++j) t.hatMinv[i][j] = T(rt.hatMinv[i * I::N + j]);
+  for (int n = 0; n < 3; ++n)
+    for (int r = 0; r < I::R; ++r)
+      for (int i = 0; i < I::N; ++i) {
+        double a = 0.0;
+        for (int j = 0; j < I::N; ++j) a += rt.hatMinv[i * I::N + j] * rt.phi1D[(n * I::R + r) * I::N + j];
+        t.Fphi[n][r][i] = T(a);
+      }
   const cudaError_t e = cudaMemcpyToSymbolAsync(itab_symbol<T, P>(), &t, sizeof(t), 0, cudaMemcpyHostToDevice, stream);
   if (e != cudaSuccess) return e;
   return cudaStreamSynchronize(stream);
@@ -465,82 +726,64 @@ struct Solver {
   ImplicitState *st;
   ImplArgs<T> args;
   size_t n;
-  int gridK, gridV, nbD;
+  int gridV;
+  static constexpr int N = IDims<P>::N;
 
   explicit Solver(dgadv_handle *hh) : h(hh), st(hh->impl) {
     n = st->n;
     args = ImplArgs<T>{};
     args.K = h->K; args.Kp = h->Kp; args.nTerms = h->nTerms;
     args.F = (const T *)h->F; args.Vn = (const T *)h->Vn; args.rhs = (const T *)h->rhs;
-    args.nbr = h->nbr; args.code = h->code;
-    gridK = (h->K + kElemThreads - 1) / kElemThreads;
+    args.nbr = h->nbr; args.code = h->code; args.A = (const T *)st->Aloc;
     gridV = (int)std::min<size_t>((n + kVecThreads - 1) / kVecThreads, 4 * 152);
-    nbD = (int)std::min<size_t>((n + kVecThreads - 1) / kVecThreads, kMaxDotBlocks);
   }
   T *vec(void *p) const { return (T *)p; }
   T *basis(int j) const { return (T *)st->V + (size_t)j * n; }
+  GridSums sums(double *out) const { return GridSums{st->partial, st->ticket, out}; }
 
   // y = ca x + cb cDot(x; t) (sources if withRhs)
   void op(const T *x, T *y, double ca, double cb, bool withRhs, double t) {
     ImplArgs<T> a = args;
     const bool rhs = withRhs && h->nTerms > 0 && h->rhs;
     for (int m = 0; m < h->nTerms; ++m) a.gco[m] = time_factor_of(h->timeFn[m], t);
-    if (rhs) k_impl_op<T, P, true><<<gridK, kElemThreads, 0, h->stream>>>(a, x, y, ca, cb);
-    else k_impl_op<T, P, false><<<gridK, kElemThreads, 0, h->stream>>>(a, x, y, ca, cb);
+    if (rhs) k_impl_op<T, P, true><<<st->blocks, dim3(kRows, N), 0, h->stream>>>(a, x, y, ca, cb);
+    else k_impl_op<T, P, false><<<st->blocks, dim3(kRows, N), 0, h->stream>>>(a, x, y, ca, cb);
   }
-  void prec(const T *r, T *z) {
-    k_impl_prec<T, P><<<gridK, kElemThreads, 0, h->stream>>>(h->K, h->Kp, (const T *)st->Pinv, r, z);
-  }
-  void build_prec(double ca, double cb) {
-    if (st->pinvVersion == h->velVersion && st->pinvA == ca && st->pinvB == cb) return;
-    k_impl_block<T, P><<<gridK, kElemThreads, 0, h->stream>>>(args, ca, cb, (T *)st->Pinv);
+  // The diagonal blocks' inverses and cDot's local part, whenever the velocity or the stage's
+  // coefficients changed.
+  int build_prec(double ca, double cb) {
+    if (st->pinvVersion == h->velVersion && st->pinvA == ca && st->pinvB == cb) return DGADV_OK;
+    int sing = 0;
+    DG_CUDA(cudaMemsetAsync(st->singular, 0, sizeof(int), h->stream));
+    k_impl_block<T, P><<<st->blocks, kRows, 0, h->stream>>>(args, ca, cb, (T *)st->Pinv, (T *)st->Aloc, st->singular);
+    DG_CUDA(cudaMemcpyAsync(&sing, st->singular, sizeof(int), cudaMemcpyDeviceToHost, h->stream));
+    DG_CUDA(cudaStreamSynchronize(h->stream));
+    if (st->ident != (sing == 0)) st->graphA = st->graphB = 0.0;   // the steps' graphs hold the other kernel
+    st->ident = sing == 0;
     st->pinvA = ca; st->pinvB = cb; st->pinvVersion = h->velVersion;
-  }
-  // dres[off + v] = <V_v, w> for v < nv (V: nv vectors of stride n)
-  void mdot(const T *V, int nv, const T *w, int off) {
-    k_mdot_n<T><<<nbD, kVecThreads, 0, h->stream>>>(V, n, nv, w, n, st->partial);
-    k_dot_final<<<nv, kVecThreads, 0, h->stream>>>(st->partial, nbD, st->dres + off);
-  }
-  // y = ay y + sgn V coef (coef in device memory)
-  void vcomb(T *y, double ay, const T *V, int nv, const double *coef, double sgn) {
-    if (nv > 0) k_vcomb_n<T><<<gridV, kVecThreads, 0, h->stream>>>(y, ay, V, n, nv, coef, sgn, n);
-  }
-  void comb(T *y, std::initializer_list<std::pair<const T *, double>> terms) {
-    Comb<T> cb{};
-    cb.nv = 0;
-    for (const auto &t : terms) { cb.x[cb.nv] = t.first; cb.c[cb.nv] = t.second; ++cb.nv; }
-    k_comb<T><<<gridV, kVecThreads, 0, h->stream>>>(y, cb, n);
+    return DGADV_OK;
   }
   void comb(T *y, const Comb<T> &cb) { k_comb<T><<<gridV, kVecThreads, 0, h->stream>>>(y, cb, n); }
-  double norm2(const T *w) {
-    mdot(w, 1, w, 0);
-    cudaMemcpyAsync(st->hres, st->dres, sizeof(double), cudaMemcpyDeviceToHost, h->stream);
-    cudaStreamSynchronize(h->stream);
-    return st->hres[0];
-  }
 
   // Arnoldi step j: w = A P^-1 v_j, orthogonalised against v_0..v_j (classical Gram-Schmidt,
-  // twice), v_{j+1} = w / |w|, and the dense update of column j.
+  // twice), v_{j+1} = w / |w|, z = P^-1 v_{j+1}, and the dense update of column j.
   void arnoldi_enqueue(int j, double ca, double cb, const GmresDense &d) {
-    const int m = st->m;
-    T *w = vec(st->w), *z = vec(st->z);
-    double *h1 = st->dres, *h2 = st->dres + (m + 1), *nw = st->dres + 2 * (m + 1);
-    prec(basis(j), z);
-    op(z, w, ca, cb, false, 0.0);
-    mdot(basis(0), j + 1, w, 0);
-    vcomb(w, 1.0, basis(0), j + 1, h1, -1.0);
-    mdot(basis(0), j + 1, w, m + 1);
-    vcomb(w, 1.0, basis(0), j + 1, h2, -1.0);
-    mdot(w, 1, w, 2 * (m + 1));
-    k_unit<T><<<gridV, kVecThreads, 0, h->stream>>>(basis(j + 1), w, nw, n);
-    k_gmres_column<<<1, 1, 0, h->stream>>>(d, h1, h2, nw, j, m);
+    const int m = st->m, nb = st->blocks;
+    const dim3 nt(kRows, N);
+    T *w = vec(st->w), *z = vec(st->z), *V = basis(0);
+    double *h1 = st->dres, *h2 = st->dres + (m + 1);
+    if (st->ident) k_arn_apply<T, P, true><<<nb, nt, 0, h->stream>>>(args, V, n, j, z, w, ca, cb, sums(h1));
+    else k_arn_apply<T, P, false><<<nb, nt, 0, h->stream>>>(args, V, n, j, z, w, ca, cb, sums(h1));
+    k_arn_first<T, N><<<nb, nt, 0, h->stream>>>(h->K, h->Kp, V, n, j, w, h1, sums(h2));
+    k_arn_second<T, N><<<nb + 1, nt, 0, h->stream>>>(h->K, h->Kp, V, n, j, w, (const T *)st->Pinv, z, h1, h2, d, m);
   }
-  // The step as a CUDA graph, captured once per j and operator (all its buffers are the
-  // handle's own; the operator's coefficients are baked in).
-  int arnoldi_step(int j, double ca, double cb, const GmresDense &d) {
-    if (h->flags & DGADV_FLAG_NO_GRAPH) {
-      arnoldi_enqueue(j, ca, cb, d);
-      return DGADV_OK;
+  // Steps j .. j + cnt - 1: kCheck of them, between two looks at the residual, as one CUDA graph captured
+  // once per j and operator (all its buffers are the handle's own; the operator's coefficients are
+  // baked in); fewer are launched directly.
+  int arnoldi_steps(int j, int cnt, double ca, double cb, const GmresDense &d) {
+    if ((h->flags & DGADV_FLAG_NO_GRAPH) || cnt != kCheck) {
+      for (int i = 0; i < cnt; ++i) arnoldi_enqueue(j + i, ca, cb, d);
+      return cudaGetLastError() == cudaSuccess ? DGADV_OK : DGADV_ECUDA;
     }
     if (st->graphA != ca || st->graphB != cb || (int)st->arnoldi.size() != st->m) {
       for (cudaGraphExec_t g : st->arnoldi)
@@ -552,7 +795,7 @@ struct Solver {
     if (!st->arnoldi[j]) {
       cudaGraph_t g = nullptr;
       if (cudaStreamBeginCapture(h->stream, cudaStreamCaptureModeThreadLocal) != cudaSuccess) return DGADV_ECUDA;
-      arnoldi_enqueue(j, ca, cb, d);
+      for (int i = 0; i < cnt; ++i) arnoldi_enqueue(j + i, ca, cb, d);
       if (cudaStreamEndCapture(h->stream, &g) != cudaSuccess) return DGADV_ECUDA;
       const cudaError_t e = cudaGraphInstantiate(&st->arnoldi[j], g, 0);
       cudaGraphDestroy(g);
@@ -567,16 +810,10 @@ struct Solver {
   // (a few iterations past convergence only improve the iterate).  Returns DGADV_OK or
   // DGADV_ENOCONV; iters accumulates iterations.
   int gmres(const T *b, T *x, double ca, double cb, double tol, int maxIter, int &iters, double &relres) {
-    constexpr int kCheck = 4;
-    const int m = st->m;
-    build_prec(ca, cb);
-    T *w = vec(st->w), *z = vec(st->z), *r = vec(st->r);
-    const double bnorm = std::sqrt(norm2(b));
-    if (bnorm == 0.0) {
-      cudaMemsetAsync(x, 0, n * sizeof(T), h->stream);
-      relres = 0.0;
-      return DGADV_OK;
-    }
+    const int m = st->m, nb = st->blocks;
+    const dim3 nt(kRows, N);
+    if (int e = build_prec(ca, cb)) return e;
+    T *z = vec(st->z), *r = vec(st->r);
     GmresDense d;
     d.H = st->dense;
     d.cs = d.H + (size_t)(m + 1) * m;
@@ -586,32 +823,34 @@ struct Solver {
     d.status = d.y + m;
     int used = 0;
     for (;;) {
-      op(x, w, ca, cb, false, 0.0);
-      comb(r, {{b, 1.0}, {w, -1.0}});
-      const double beta = std::sqrt(norm2(r));
-      relres = beta / bnorm;
+      k_impl_residual<T, P><<<nb, nt, 0, h->stream>>>(args, b, x, r, ca, cb, sums(st->dres));
+      cudaMemcpyAsync(st->hres, st->dres, 2 * sizeof(double), cudaMemcpyDeviceToHost, h->stream);
+      if (cudaStreamSynchronize(h->stream) != cudaSuccess) return DGADV_ECUDA;
+      const double bnorm = std::sqrt(st->hres[1]);
+      if (bnorm == 0.0) {
+        cudaMemsetAsync(x, 0, n * sizeof(T), h->stream);
+        relres = 0.0;
+        return DGADV_OK;
+      }
+      relres = std::sqrt(st->hres[0]) / bnorm;
       if (relres <= tol) return DGADV_OK;
       if (used >= maxIter) return DGADV_ENOCONV;
-      k_unit<T><<<gridV, kVecThreads, 0, h->stream>>>(basis(0), r, st->dres, n);
-      k_gmres_start<<<1, 1, 0, h->stream>>>(d, st->dres, m);
+      k_arn_start<T, N><<<nb, nt, 0, h->stream>>>(h->K, h->Kp, r, basis(0), (const T *)st->Pinv, z, st->dres, d, m);
       int j = 0;
       while (j < m && used < maxIter) {
-        ++used;
-        ++iters;
-        if (int e = arnoldi_step(j, ca, cb, d)) return e;
-        ++j;
-        if (j % kCheck == 0 || j == m || used >= maxIter) {
-          cudaMemcpyAsync(st->hres, d.status, 3 * sizeof(double), cudaMemcpyDeviceToHost, h->stream);
-          if (cudaStreamSynchronize(h->stream) != cudaSuccess) return DGADV_ECUDA;
-          relres = st->hres[0] / bnorm;
-          if (relres <= tol || st->hres[2] != 0.0) break;
-        }
+        const int cnt = std::min(std::min(kCheck, m - j), maxIter - used);
+        if (int e = arnoldi_steps(j, cnt, ca, cb, d)) return e;
+        used += cnt;
+        iters += cnt;
+        j += cnt;
+        cudaMemcpyAsync(st->hres, d.status, 3 * sizeof(double), cudaMemcpyDeviceToHost, h->stream);
+        if (cudaStreamSynchronize(h->stream) != cudaSuccess) return DGADV_ECUDA;
+        relres = st->hres[0] / bnorm;
+        if (relres <= tol || st->hres[2] != 0.0) break;
       }
       // x += P^-1 V y with y = H^-1 g over the columns in use
-      k_gmres_solve<<<1, 1, 0, h->stream>>>(d, m);
-      vcomb(r, 0.0, basis(0), j, d.y, 1.0);
-      prec(r, z);
-      comb(x, {{x, 1.0}, {z, 1.0}});
+      k_gmres_solve<<<1, 256, 0, h->stream>>>(d, m);
+      k_arn_update<T, N><<<nb, nt, 0, h->stream>>>(h->K, h->Kp, basis(0), n, j, d.y, (const T *)st->Pinv, x);
     }
   }
 
@@ -622,7 +861,9 @@ struct Solver {
     if (!S) { h->err = "DIRK order must be 1..4"; return DGADV_EINVAL; }
     T *cn = (T *)h->cn, *x = vec(st->x), *rhs = vec(st->b), *s = vec(st->s);
     const T *zero = vec(st->zero);
+    const bool sources = h->nTerms > 0 && h->rhs;
     worst = 0.0;
+    if (int e = build_prec(1.0, -tau * a[0][0])) return e;   // the operator needs the local part
     for (int nn = 0; nn < nSteps; ++nn) {
       const double t0 = (double)(nStep0 + nn) * tau;
       cudaMemcpyAsync(x, cn, n * sizeof(T), cudaMemcpyDeviceToDevice, h->stream);
@@ -630,12 +871,12 @@ struct Solver {
         double ci = 0.0;
         for (int j = 0; j <= i; ++j) ci += a[i][j];
         const double ti = t0 + ci * tau, gam = tau * a[i][i];
-        op(zero, s, 0.0, 1.0, true, ti);                 // s_i = M^-1 sysV(t_i)
+        if (sources) op(zero, s, 0.0, 1.0, true, ti);    // s_i = M^-1 sysV(t_i)
         Comb<T> cb{};
         cb.nv = 0;
         cb.x[cb.nv] = cn; cb.c[cb.nv++] = 1.0;
         for (int j = 0; j < i; ++j) { cb.x[cb.nv] = (const T *)st->kst + (size_t)j * n; cb.c[cb.nv++] = tau * a[i][j]; }
-        cb.x[cb.nv] = s; cb.c[cb.nv++] = gam;
+        if (sources) { cb.x[cb.nv] = s; cb.c[cb.nv++] = gam; }
         comb(rhs, cb);
         double rr = 0.0;
         const int e = gmres(rhs, x, 1.0, -gam, tol, maxIter, iters, rr);
@@ -650,6 +891,7 @@ struct Solver {
 
   int stationary(double tol, int maxIter, int &iters, double &res) {
     T *cn = (T *)h->cn, *s = vec(st->s);
+    if (int e = build_prec(0.0, -1.0)) return e;
     op(vec(st->zero), s, 0.0, 1.0, true, 0.0);         // M^-1 sysV
     const int e = gmres(s, cn, 0.0, -1.0, tol, maxIter, iters, res);   // M^-1 A x = M^-1 sysV
     if (e) return e;
@@ -677,9 +919,13 @@ int ensure_state(dgadv_handle *h, int restart) {
     if ((e = dev_alloc(h, b, vb))) return e;
   if ((e = dev_alloc(h, &st->kst, 4 * vb))) return e;
   if ((e = dev_alloc(h, &st->Pinv, (size_t)h->N * h->N * h->Kp * rb))) return e;
-  if ((e = dev_alloc(h, (void **)&st->partial, (size_t)(restart + 2) * kMaxDotBlocks * 8))) return e;
-  if ((e = dev_alloc(h, (void **)&st->dres, (size_t)3 * (restart + 1) * 8))) return e;
-  if ((e = dev_alloc(h, (void **)&st->dcoef, (size_t)(restart + 1) * 8))) return e;
+  if ((e = dev_alloc(h, &st->Aloc, (size_t)h->N * h->N * h->Kp * rb))) return e;
+  st->blocks = (h->K + kRows - 1) / kRows;
+  if ((e = dev_alloc(h, (void **)&st->partial, (size_t)(restart + 2) * st->blocks * 8))) return e;
+  if ((e = dev_alloc(h, (void **)&st->ticket, 16))) return e;
+  if ((e = dev_alloc(h, (void **)&st->singular, 16))) return e;
+  if ((e = dev_alloc(h, (void **)&st->dres, (size_t)(2 * restart + 3) * 8))) return e;
+  DG_CUDA(cudaMemsetAsync(st->ticket, 0, 16, h->stream));
   if ((e = dev_alloc(h, (void **)&st->dense, ((size_t)(restart + 1) * restart + 4 * (size_t)restart + 8) * 8))) return e;
   DG_CUDA(cudaMallocHost((void **)&st->hres, (size_t)3 * (restart + 1) * 8));
   DG_CUDA(cudaMemsetAsync(st->V, 0, (size_t)(restart + 1) * vb, h->stream));
