@@ -119,6 +119,7 @@ struct dgadv_handle {
   // discrete adjoint (dgadv_forward_record / dgadv_backward)
   int nModes = 0;
   double *modeF = nullptr, *modeV = nullptr;   // nModes x 2Q x Kp, nModes x 3R x Kp (FP64)
+  double *velTmp = nullptr;                    // combined velocity factors in FP64, and theta
   void *adjSlots = nullptr;                    // state snapshots, nSlots x N x Kp
   void *adjStages = nullptr;                   // stage states c^(1..S-1) of every step (or null)
   int adjStageSteps = 0;
