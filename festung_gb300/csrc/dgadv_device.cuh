@@ -709,7 +709,7 @@ __device__ __forceinline__ void stage_expect(uint64_t *bar, int nT, int nI) {
 // kernel at most waits beside the running one.  Triggered before the wait, a whole chain of small
 // kernels piles up on the SMs, each placed where the ones before it left room: their blocks end up
 // on few SMs, and a chain can run slower than without the early launch (four species on 8192
-// triangles, p = 1, FP64: 123 us per step so, 43 us now; 6498 triangles, p = 2, FP64: 45 and 23.5 us
+// triangles, p = 1, FP64: 123 us per step so, 50 us now; 6498 triangles, p = 2, FP64: 45 and 23.5 us
 // per stage, 30 without dependent launch).
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
@@ -1101,6 +1101,10 @@ struct StageScalars {
   int *flag;            // bit 0: non-finite value seen; bit 1: a bounded wait timed out
 };
 
+// Basis functions of x1 alone (1, x1, x1^2 and x1^3 rows of the hierarchical basis): their derivative
+// in x2 is zero, as is the first function's in x1, and the volume term leaves these products out.
+__host__ __device__ constexpr bool basis_in_x1(int i) { return i == 0 || i == 1 || i == 3 || i == 6; }
+
 // Operator variants of the stage kernel (VAR):
 //   kOpPlain    volume term at the quadrature points, upwind flux at the edge points;
 //   kOpFp32     (double-float state only) the operator (volume, flux, hatM^-1 = I) in FP32
@@ -1128,6 +1132,12 @@ __device__ __forceinline__ void stage_op_tile(const Geo<T> g, const T *cin, cons
   // with the mass solve (FP64, double-float) and no source terms, hatM^-1 is folded into the
   // test-function tables of the volume and flux terms (Fg1, Fg2, Fphi)
   constexpr bool kFold = sizeof(A) == 8 && !RHS;
+  // FP32 issues too many instructions to be bound by memory: 1090 per warp at p = 2, of which 243 are
+  // floating point.  So every neighbour comes from global memory (the block's own lines are in
+  // L1 or L2) instead of a choice between two memories per edge, and the upwind flux branches per edge
+  // instead of per point.  131072 triangles, p = 2, 60 steps with input and output: 3.56 -> 3.41 ms;
+  // 24 instances: 5.93 -> 5.66 ms; 524288 triangles, p = 3, hierarchical, 8 steps: 4.69 -> 4.65 ms.
+  constexpr bool kLean = std::is_same_v<T, float>;
   constexpr int NT = StageRows<T, P>::op(MODE, LIN, EOP);
   extern __shared__ __align__(128) unsigned char smem[];
   uint64_t *bar = (uint64_t *)(smem + StageRows<T, P>::bar_offset(NT, 1, blockDim.x));
@@ -1194,6 +1204,12 @@ __device__ __forceinline__ void stage_op_tile(const Geo<T> g, const T *cin, cons
   A cn[3][N];
 #pragma unroll
   for (int n = 0; n < 3; ++n) {
+    if constexpr (kLean) {                        // without a neighbour: any element, not used
+      const T *pn = cin + (nb[n] >= 0 ? nb[n] : k0);
+#pragma unroll
+      for (int j = 0; j < N; ++j) cn[n][j] = as_arith<A>(pn[(size_t)j * Kp]);
+      continue;
+    }
     const bool outside = nb[n] >= 0 && (nb[n] < k0 || nb[n] >= k0 + eb);
 #pragma unroll
     for (int j = 0; j < N; ++j) cn[n][j] = outside ? as_arith<A>(cin[(size_t)j * Kp + nb[n]]) : A(0);
@@ -1207,11 +1223,13 @@ __device__ __forceinline__ void stage_op_tile(const Geo<T> g, const T *cin, cons
     Acc<A> rhs[N];
 #pragma unroll
     for (int i = 0; i < N; ++i) { c[i] = as_arith<A>(srow<T>(smem, rC + i)[t]); rhs[i] = Acc<A>(A(0)); }
+    if constexpr (!kLean) {
 #pragma unroll
     for (int n = 0; n < 3; ++n)
       if (nb[n] >= k0 && nb[n] < k0 + eb)
 #pragma unroll
         for (int j = 0; j < N; ++j) cn[n][j] = as_arith<A>(srow<T>(smem, rC + j)[nb[n] - k0]);
+    }
     bool summed = false;   // cdot is done in fixed point; else the FP64 rows come from global memory
     if constexpr (FXP)
       summed = fx::element_cdot<P>(fx_tab<P>(), (const Dig *)srow<T>(smem, rF) + t, (const Dig *)srow<T>(smem, rV) + t,
@@ -1243,7 +1261,10 @@ __device__ __forceinline__ void stage_op_tile(const Geo<T> g, const T *cin, cons
       const T(&G1)[Q][N] = kFold ? tb.Fg1 : tb.g1;
       const T(&G2)[Q][N] = kFold ? tb.Fg2 : tb.g2;
 #pragma unroll
-      for (int i = 0; i < N; ++i) { rhs[i].fma(as_arith<A>(G1[qq][i]), f1); rhs[i].fma(as_arith<A>(G2[qq][i]), f2); }
+      for (int i = 0; i < N; ++i) {
+        if (kFold || i != 0) rhs[i].fma(as_arith<A>(G1[qq][i]), f1);
+        if (kFold || !basis_in_x1(i)) rhs[i].fma(as_arith<A>(G2[qq][i]), f2);
+      }
     }
     }
     // upwind edge term (with the element operator: the inflow terms only)
@@ -1252,6 +1273,40 @@ __device__ __forceinline__ void stage_op_tile(const Geo<T> g, const T *cin, cons
     for (int n = 0; n < 3; ++n) {
       const int np = (code >> (2 * n)) & 3;
       const bool outOk = !EOP && ((code >> (6 + n)) & 1);
+      if constexpr (kLean) {
+        A v[R], tr[R];
+        bool out = false, in = false;
+#pragma unroll
+        for (int r2 = 0; r2 < R; ++r2) {
+          v[r2] = srow<T>(smem, rV + n * R + r2)[t];
+          tr[r2] = A(0);
+          out |= v[r2] > A(0);
+          in |= v[r2] < A(0);
+        }
+        if (out && outOk)
+#pragma unroll
+          for (int r2 = 0; r2 < R; ++r2) {
+            Acc<A> s(A(0));
+#pragma unroll
+            for (int j = 0; j < N; ++j) s.fma(tb.phi1D[n][r2][j], c[j]);
+            if (v[r2] > A(0)) tr[r2] = s.get();
+          }
+        if (in && nb[n] >= 0)
+#pragma unroll
+          for (int r2 = 0; r2 < R; ++r2) {
+            Acc<A> s(A(0));
+#pragma unroll
+            for (int j = 0; j < N; ++j) s.fma(tb.thetaPhi[n][np][r2][j], cn[n][j]);
+            if (v[r2] < A(0)) tr[r2] = s.get();
+          }
+#pragma unroll
+        for (int r2 = 0; r2 < R; ++r2) {
+          const A fl = v[r2] * tr[r2];
+#pragma unroll
+          for (int i = 0; i < N; ++i) rhs[i].fms(tb.phi1D[n][r2][i], fl);
+        }
+        continue;
+      }
 #pragma unroll
       for (int r2 = 0; r2 < R; ++r2) {
         const A v = as_arith<A>(FXP ? g.Vn[(size_t)(n * R + r2) * Kp + k] : srow<T>(smem, rV + n * R + r2)[t]);
