@@ -1258,12 +1258,11 @@ __device__ __forceinline__ void stage_op_tile(const Geo<T> g, const T *cin, cons
       const A cq = cqa.get();
       const A f1 = as_arith<A>(srow<T>(smem, rF + qq)[t]) * cq;
       const A f2 = as_arith<A>(srow<T>(smem, rF + Q + qq)[t]) * cq;
-      const T(&G1)[Q][N] = kFold ? tb.Fg1 : tb.g1;
-      const T(&G2)[Q][N] = kFold ? tb.Fg2 : tb.g2;
+      const T *G1 = kFold ? tb.Fg1[qq] : tb.g1[qq], *G2 = kFold ? tb.Fg2[qq] : tb.g2[qq];
 #pragma unroll
       for (int i = 0; i < N; ++i) {
-        if (kFold || i != 0) rhs[i].fma(as_arith<A>(G1[qq][i]), f1);
-        if (kFold || !basis_in_x1(i)) rhs[i].fma(as_arith<A>(G2[qq][i]), f2);
+        if (kFold || i != 0) rhs[i].fma(as_arith<A>(G1[i]), f1);
+        if (kFold || !basis_in_x1(i)) rhs[i].fma(as_arith<A>(G2[i]), f2);
       }
     }
     }
