@@ -98,8 +98,8 @@ enum {
                                    sets of work states and limiter records (and with 3 the
                                    limiter's key sets), allocated by dgadv_forward_record.
                                    Gradients bitwise unchanged                                 */
-  DGADV_OPT_ELEMENT_OPERATOR = 10, /* FP64 and double-float handles without source terms (and,
-                                   double-float, without the FP32 operator): 1 (default) keeps the
+  DGADV_OPT_ELEMENT_OPERATOR = 10, /* FP64 handles, and double-float handles without source terms
+                                   and without the FP32 operator: 1 (default) keeps the
                                    stage operator's volume term and the element's own outflow
                                    terms as one N x N matrix per element (N^2 reals per element,
                                    rebuilt whenever the velocity changes), which takes the FP64
