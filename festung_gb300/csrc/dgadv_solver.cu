@@ -229,20 +229,25 @@ static int create_impl(const dgadv_mesh *mesh, const dgadv_params *prm, const st
   // the vertices of each block of kBlock elements, and the elements' positions in their block's list
   std::vector<int> vtPtr(1, 0), vtIdx;
   std::vector<unsigned short> vtLoc(3 * (size_t)Kp, 0);
-  for (int b = 0; b < Kp; b += kBlock) {
-    std::vector<int> v;
-    for (int k = b; k < std::min(b + kBlock, K); ++k)
-      for (int n = 0; n < 3; ++n) v.push_back(V0T[(size_t)n * Kp + k]);
-    std::sort(v.begin(), v.end());
-    v.erase(std::unique(v.begin(), v.end()), v.end());
-    for (int k = b; k < std::min(b + kBlock, K); ++k)
-      for (int n = 0; n < 3; ++n)
-        vtLoc[(size_t)n * Kp + k] = (unsigned short)(std::lower_bound(v.begin(), v.end(), V0T[(size_t)n * Kp + k]) - v.begin());
-    vtIdx.insert(vtIdx.end(), v.begin(), v.end());
-    vtPtr.push_back((int)vtIdx.size());
-    h->vtMax = std::max(h->vtMax, (int)v.size());
+  if (h->lim) {                                     // the limiter's kernels alone use them
+    std::vector<int> seen(h->numV, -1), at(h->numV), v;   // the last block with the vertex, its place there
+    for (int b = 0; b < Kp; b += kBlock) {
+      v.clear();
+      const int end = std::min(b + kBlock, K);
+      for (int k = b; k < end; ++k)
+        for (int n = 0; n < 3; ++n) {
+          const int w = V0T[(size_t)n * Kp + k];
+          if (seen[w] != b) { seen[w] = b; v.push_back(w); }
+        }
+      std::sort(v.begin(), v.end());
+      for (size_t i = 0; i < v.size(); ++i) at[v[i]] = (int)i;
+      for (int k = b; k < end; ++k)
+        for (int n = 0; n < 3; ++n) vtLoc[(size_t)n * Kp + k] = (unsigned short)at[V0T[(size_t)n * Kp + k]];
+      vtIdx.insert(vtIdx.end(), v.begin(), v.end());
+      vtPtr.push_back((int)vtIdx.size());
+      h->vtMax = std::max(h->vtMax, (int)v.size());
+    }
   }
-  if (!h->lim) h->vtMax = 0;   // the limiter's kernels alone use them
   // CSR vertex -> elements (internal ids)
   std::vector<int> vptr(h->numV + 1, 0), vidx(3 * (size_t)K);
   for (int k = 0; k < K; ++k)
