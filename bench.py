@@ -905,8 +905,9 @@ def run_ours(args):
     roof['note'] = ('L2-resident: the bytes a FP64 stage touches on this mesh (about 120 MB cold per '
                     'stage with the element operator, traffic) fit the 129 MB L2 for the most part, so '
                     'they are served mostly from L2 once a solve runs; the FP64 kernels are bound '
-                    'by GB300\'s FP64 rate, not by bandwidth (fp64_rate); the HBM-bound figure is hbm_case')
-    # the bound that applies: the FP64 pipe, against cuBLAS DGEMM on the same GPU
+                    'by instruction issue and latency, not by bandwidth (their sums run in fixed point on '
+                    'the integer units, fp64_rate); the HBM-bound figure is hbm_case')
+    # the FP64 operations they stand for, against cuBLAS DGEMM on the same GPU
     peak64 = fp64_peak()
     rate = {'peak_tflops': peak64, 'peak_source': 'measured: cuBLAS DGEMM 4096^3 (torch.matmul float64)',
             'kernels': {}}
