@@ -816,12 +816,7 @@ __device__ __forceinline__ void patch_minmax(const LimIn<T> &, const PatchView<T
 }
 // The extremes alone (no boundary data).
 template <typename T>
-__device__ __forceinline__ void patch_extremes(const LimIn<T> &li, const VKeys<T, 1> &kv, const T *sh, T mn[3], T mx[3]) {
-  const T none[3] = {T(NAN), T(NAN), T(NAN)};
-  patch_minmax<T, 1>(li, kv, sh, 0, none, mn, mx);
-}
-template <typename T>
-__device__ __forceinline__ void patch_extremes(const LimIn<T> &, const PatchView<T> &kv, const T *, T mn[3], T mx[3]) {
+__device__ __forceinline__ void patch_extremes(const PatchView<T> &kv, T mn[3], T mx[3]) {
 #pragma unroll
   for (int n = 0; n < 3; ++n) { mn[n] = kv.pv[kv.l[n]]; mx[n] = kv.pv[kv.stride + kv.l[n]]; }
 }
@@ -1175,10 +1170,10 @@ __device__ __forceinline__ void stage_op_tile(const Geo<T> g, const T *cin, cons
   if (MODE != 0 && active) load_vertices(g, k, vt, vid);
   VtList vl{0, 0, 0};
   if (vt && staged) vl = vt_list(g, tile);
-  int ax = 0;
+  fx::OpExp<P> ax;
   T src[N];                                       // the source terms at this stage's time
   if constexpr (FXP) {                            // neighbours across inflow edges only
-    if (active) ax = g.aopE[k];
+    if (active) ax.load(g.aopE, Kp, k);
     if (g.rhsM) {
 #pragma unroll
       for (int i = 0; i < N; ++i) src[i] = T(0);
@@ -1190,7 +1185,7 @@ __device__ __forceinline__ void stage_op_tile(const Geo<T> g, const T *cin, cons
     }
 #pragma unroll
     for (int n = 0; n < 3; ++n)
-      if (!((ax >> (22 + n)) & 1)) nb[n] = -1;
+      if (active && !ax.inflow(n)) nb[n] = -1;
   }
   pdl_wait();
   pdl_trigger();
@@ -1874,8 +1869,8 @@ __device__ __forceinline__ void limit_dot_lin_tile(const Geo<T> g, const T *cin,
   if (active) load_vertices(g, k, true, vid);
   VtList vl{0, 0, 0};
   if (staged) vl = vt_list(g, tile);
-  int mx = -1;
-  if (fxOn && active) mx = g.mtE[k];
+  fx::CorrExp<P> mx;
+  if (fxOn && active) mx.load(g.mtE, Kp, k);
   pdl_wait();
   pdl_trigger();
   reset_next<T>(g, lo, k, nTiles < 0 ? -1 : tile, nTiles);
@@ -1897,11 +1892,12 @@ __device__ __forceinline__ void limit_dot_lin_tile(const Geo<T> g, const T *cin,
 #pragma unroll
     for (int i = 0; i < N; ++i) cd[i] = srow<T>(smem, rD + i)[t];
     bool limited = false;   // cd is done in fixed point
-    if constexpr (std::is_same_v<T, double>)
+    if constexpr (std::is_same_v<T, double> && P >= 2)
       if (fxOn) {
         T lo3[3], hi3[3];
-        patch_extremes(li, pv, sh, lo3, hi3);
-        limited = fx::linear_cdot_limit<P>(fx_tab<P>(), lo3, hi3, (const Dig *)srow<T>(smem, rQ) + t, kBlock, mx, cd);
+        patch_extremes(pv, lo3, hi3);
+        limited = fx::linear_cdot_limit<P>(fx_tab<P>(), lo3, hi3, (const Dig *)srow<T>(smem, rQ) + t, kBlock, mx,
+                                           lin_mean<T, P>(cd), cd);
       }
     if (!limited) {
     lin_u3<T, P>(cd, u);
@@ -1969,21 +1965,18 @@ k_limit_dot_lin(const Geo<T> g, const T *cin, const T *c0, const T *tbuf,
   limit_dot_lin_tile<T, P>(g, cin, c0, tbuf, out, li, lo, sc, blockIdx.x);
 }
 
-// One element's coefficients limited in place (FX: FP64 sums in fixed point).
+// One element's coefficients limited in place (FX: FP64 sums in fixed point, for kv in the block's table).
 template <typename T, int P, bool FX, typename KV>
 __device__ __forceinline__ void limit_lin_element(const LimIn<T> &li, const KV &kv, const T *sh, int dmask,
                                                   const T data[3], T *c) {
   constexpr int N = Dims<P>::N, NQ = 1;
   const Tab<T, P> &tb = tab<T, P>();
+  if constexpr (FX && std::is_same_v<T, double> && P >= 1) {
+    T lo3[3], hi3[3];
+    patch_extremes(kv, lo3, hi3);
+    if (fx::linear_limit<P>(fx_tab<P>(), lo3, hi3, dmask, data, lin_mean<T, P>(c), c)) return;
+  }
   T u[N], du[N];
-  bool limited = false;   // c is done in fixed point
-  if constexpr (FX && std::is_same_v<T, double>)
-    {
-      T lo3[3], hi3[3];
-      patch_extremes(li, kv, sh, lo3, hi3);
-      limited = fx::linear_limit<P>(fx_tab<P>(), lo3, hi3, dmask, data, c);
-    }
-  if (!limited) {
   lin_u3<T, P>(c, u);
   if (lin_alpha<T, P, NQ>(li, kv, sh, u, dmask, data, du)) {
     // limited: u - du is the linear Taylor polynomial (u_0, alpha u_1, alpha u_2); back in the
@@ -1999,7 +1992,6 @@ __device__ __forceinline__ void limit_lin_element(const LimIn<T> &li, const KV &
       }
       c[i] = s.get();
     }
-  }
   }
 }
 

@@ -52,23 +52,30 @@ template <typename T, int P> struct Tab {
   T Fphi[3][R][N];
 };
 
-// One factor of a fixed-point sum (dgadv_fixed.cuh): h 2^29 + l.
+// One factor of a fixed-point sum (dgadv_fixed.cuh): h 2^31 + l.
 struct alignas(8) Dig {
   int h, l;
 };
 // Tables of the FP64 stage kernels in digits, each entry scaled so that the sums it enters stay
-// below 1: thetaPhi by 2^-eT (the largest row sum over j), Fphi by 2^-eF (the largest sum over the
-// nine or so edge points), row i of DM by 2^-eDM[i] (its sum), row i of DMi, the first three
-// columns of DM^-1 with column j times 2^eDM[j], by 2^-eDMi[i].
+// below 1: thetaPhi by 2^-eT (the largest row sum over j), row i of an edge's Fphi by 2^-eF[n][i] (its sum over
+// the points), row i of DM by 2^-eDM[i][.], order by order, and of
+// DM^-1's first three columns by 2^-eDMi[i][.].
 template <int P> struct FxTab {
   static constexpr int N = Dims<P>::N, R = Dims<P>::R;
   Dig thetaPhi[3][3][R][N];
   Dig Fphi[3][R][N];
   Dig DM[N][N];
   Dig DMi[N][3];
-  int eT, eF;
-  int eDM[N < 3 ? 3 : N], eDMi[N];
+  int eT, eF[3][N];
+  int eDM[N][P + 1], eDMi[N][2];
 };
+
+// 32-bit words per element of the digits' exponents: the element operator's (one byte per row and part
+// of the coefficients, and per edge) and the linear limiter's correction rows' (one per row and
+// order of the derivatives), after a head word (fx::OpExp, fx::CorrExp).
+constexpr int op_parts(int p) { return p == 0 ? 1 : 2; }
+constexpr int op_exp_words(int p) { return 1 + (op_parts(p) * ((p + 1) * (p + 2) / 2) + 3 + 3) / 4; }
+constexpr int corr_exp_words(int p) { return 1 + (p * ((p + 1) * (p + 2) / 2) + 3) / 4; }
 
 // Static per-element data of one mesh (device pointers, SoA with stride Kp).
 template <typename T> struct Geo {
@@ -100,7 +107,7 @@ template <typename T> struct Geo {
   int timeFn[4];
   const int *instOf; // ensembles: instance of each block of kBlock elements (null: one instance)
   // FP64 in fixed point (null: FP64 arithmetic): digits of Aop, Vn and the linear limiter's MT, and
-  // their exponents per element
+  // their exponents (op_exp_words x Kp, corr_exp_words x Kp)
   const Dig *AopX, *VnX, *MTX;
   const int *aopE, *mtE;
   const T *rhsM;     // FP64: rhs with hatM^-1 applied, for the element operator (null without terms)

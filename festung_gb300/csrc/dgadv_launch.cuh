@@ -6,135 +6,18 @@
 #include <string>
 
 #include "dgadv_device.cuh"
+#include "dgadv_tables.h"
 
 namespace dgadv {
-
-// A table entry x 2^-E as digits, to the nearest.
-static Dig host_digits(double x, int E) {
-  const long long X = std::llrint(std::ldexp(x, fx::kW - E));
-  Dig d;
-  d.l = (int)((uint32_t)X << 3) >> 3;
-  d.h = (int)((X - d.l) >> 29);
-  return d;
-}
-// The least E with x <= 2^E.
-static int host_exponent(double x) {
-  int e = 0;
-  if (x > 0.0 && std::frexp(x, &e) == 0.5) --e;
-  return e;
-}
-// The digit tables (FxTab) from the FP64 tables.
-template <int P>
-static cudaError_t upload_digits(const Tab<double, P> &t) {
-  constexpr int N = Dims<P>::N, R = Dims<P>::R;
-  FxTab<P> f;
-  double rowT = 0.0, sumF = 0.0;
-  for (int n = 0; n < 3; ++n)
-    for (int np = 0; np < 3; ++np)
-      for (int r = 0; r < R; ++r) {
-        double s = 0.0;
-        for (int j = 0; j < N; ++j) s += std::fabs(t.thetaPhi[n][np][r][j]);
-        rowT = std::max(rowT, s);
-      }
-  for (int i = 0; i < N; ++i) {
-    double s = 0.0;
-    for (int n = 0; n < 3; ++n)
-      for (int r = 0; r < R; ++r) s += std::fabs(t.Fphi[n][r][i]);
-    sumF = std::max(sumF, s);
-  }
-  f.eT = host_exponent(rowT);
-  f.eF = host_exponent(sumF);
-  for (int n = 0; n < 3; ++n)
-    for (int r = 0; r < R; ++r)
-      for (int i = 0; i < N; ++i) {
-        f.Fphi[n][r][i] = host_digits(t.Fphi[n][r][i], f.eF);
-        for (int np = 0; np < 3; ++np) f.thetaPhi[n][np][r][i] = host_digits(t.thetaPhi[n][np][r][i], f.eT);
-      }
-  for (int i = 0; i < (N < 3 ? 3 : N); ++i) {
-    double s = 0.0;
-    for (int j = 0; i < N && j < N; ++j) s += std::fabs(t.DM[i][j]);
-    f.eDM[i] = host_exponent(s);
-    for (int j = 0; i < N && j < N; ++j) f.DM[i][j] = host_digits(t.DM[i][j], f.eDM[i]);
-  }
-  for (int i = 0; i < N; ++i) {
-    double c[3], s = 0.0;
-    for (int j = 0; j < 3; ++j) {
-      c[j] = j < N ? std::ldexp(t.DMinv[i][j], f.eDM[j]) : 0.0;
-      s += std::fabs(c[j]);
-    }
-    f.eDMi[i] = host_exponent(s);
-    for (int j = 0; j < 3; ++j) f.DMi[i][j] = host_digits(c[j], f.eDMi[i]);
-  }
-  return cudaMemcpyToSymbol(fx_symbol<P>(), &f, sizeof(f));
-}
 
 template <typename T, int P, bool DIGITS = std::is_same_v<T, double>>
 static cudaError_t upload_tables(const RefTables &rt) {
   Tab<T, P> t;
-  constexpr int N = Dims<P>::N, Q = Dims<P>::Q, R = Dims<P>::R;
-  for (int q = 0; q < Q; ++q)
-    for (int i = 0; i < N; ++i) {
-      t.phiQ[q][i] = T(rt.phiQ[q * N + i]);
-      t.g1[q][i] = T(rt.gradQ[q * N + i]);
-      t.g2[q][i] = T(rt.gradQ[Q * N + q * N + i]);
-    }
-  for (int n = 0; n < 3; ++n)
-    for (int r = 0; r < R; ++r)
-      for (int i = 0; i < N; ++i) t.phi1D[n][r][i] = T(rt.phi1D[(n * R + r) * N + i]);
-  for (int nn = 0; nn < 3; ++nn)
-    for (int np = 0; np < 3; ++np)
-      for (int r = 0; r < R; ++r)
-        for (int i = 0; i < N; ++i) t.thetaPhi[nn][np][r][i] = T(rt.thetaPhi[((nn * 3 + np) * R + r) * N + i]);
-  for (int i = 0; i < N; ++i)
-    for (int j = 0; j < N; ++j) {
-      t.hatMinv[i][j] = T(rt.hatMinv[i * N + j]);
-      t.DM[i][j] = T(rt.DM[i * N + j]);
-      t.DMinv[i][j] = T(rt.DMinv[i * N + j]);
-    }
-  // Gr = DM^-T hatM DM^-1 in FP64, then rounded
-  for (int i = 0; i < N; ++i)
-    for (int j = 0; j < N; ++j) {
-      double s = 0.0;
-      for (int a = 0; a < N; ++a) {
-        double r = 0.0;
-        for (int b = 0; b < N; ++b) r += rt.hatM[a * N + b] * rt.DMinv[b * N + j];
-        s += rt.DMinv[a * N + i] * r;
-      }
-      t.Gr[i][j] = T(s);
-    }
-  // adjoint tables (the forward FP32 path takes hatM^-1 = I; so does its adjoint)
-  const bool massSolve = sizeof(T) == 8;
-  auto fold = [&](const double *row, int j) {
-    if (!massSolve) return row[j];
-    double a = 0.0;
-    for (int i = 0; i < N; ++i) a += row[i] * rt.hatMinv[i * N + j];
-    return a;
-  };
-  for (int q = 0; q < Q; ++q)
-    for (int j = 0; j < N; ++j) {
-      t.Hg1[q][j] = T(fold(&rt.gradQ[q * N], j));
-      t.Hg2[q][j] = T(fold(&rt.gradQ[Q * N + q * N], j));
-    }
-  for (int n = 0; n < 3; ++n)
-    for (int r = 0; r < R; ++r)
-      for (int j = 0; j < N; ++j) t.Hphi[n][r][j] = T(fold(&rt.phi1D[(n * R + r) * N], j));
-  // forward tables: hatM^-1 applied from the left, in FP64, then rounded
-  auto lfold = [&](const double *row, int i) {
-    if (!massSolve) return row[i];
-    double a = 0.0;
-    for (int j = 0; j < N; ++j) a += rt.hatMinv[i * N + j] * row[j];
-    return a;
-  };
-  for (int q = 0; q < Q; ++q)
-    for (int i = 0; i < N; ++i) {
-      t.Fg1[q][i] = T(lfold(&rt.gradQ[q * N], i));
-      t.Fg2[q][i] = T(lfold(&rt.gradQ[Q * N + q * N], i));
-    }
-  for (int n = 0; n < 3; ++n)
-    for (int r = 0; r < R; ++r)
-      for (int i = 0; i < N; ++i) t.Fphi[n][r][i] = T(lfold(&rt.phi1D[(n * R + r) * N], i));
+  fill_tables(rt, t);
   if constexpr (DIGITS) {
-    const cudaError_t e = upload_digits<P>(t);
+    FxTab<P> f;
+    fill_digit_tables(t, f);
+    const cudaError_t e = cudaMemcpyToSymbol(fx_symbol<P>(), &f, sizeof(f));
     if (e != cudaSuccess) return e;
   }
   return cudaMemcpyToSymbol(tab_symbol<T, P>(), &t, sizeof(t));

@@ -13,6 +13,7 @@
 #include <string>
 #include <vector>
 
+#include "dgadv_kernels.cuh"
 #include "dgadv_handle.h"
 
 namespace dgadv {
@@ -368,9 +369,10 @@ static int create_impl(const dgadv_mesh *mesh, const dgadv_params *prm, const st
   if (ops(h).fix_correction && h->limdot && h->limType == DGADV_LIM_LINEAR) {
     const size_t nQ = (size_t)N * (N - 1) * Kp * 8;
     if ((st = dev_alloc(h, &h->MTX, nQ))) return st;
-    if ((st = dev_alloc(h, (void **)&h->mtE, (size_t)Kp * 4))) return st;
+    const size_t nE = (size_t)corr_exp_words(h->p) * Kp * 4;
+    if ((st = dev_alloc(h, (void **)&h->mtE, nE))) return st;
     DG_CUDA(cudaMemset(h->MTX, 0, nQ));
-    DG_CUDA(cudaMemset(h->mtE, 0, (size_t)Kp * 4));
+    DG_CUDA(cudaMemset(h->mtE, 0, nE));
     DG_CUDA(ops(h).fix_correction(h));
   }
   DG_CUDA(cudaDeviceSynchronize());
@@ -763,7 +765,7 @@ int dgadv::refresh_element_operator(dgadv_handle *h) {
     if ((st = dev_alloc(h, &h->Aop, (size_t)h->N * h->N * h->Kp * o.realBytes))) return st;
     DG_CUDA(cudaMemset(h->Aop, 0, (size_t)h->N * h->N * h->Kp * o.realBytes));
     if (h->prec == DGADV_FP64) {   // its digits (padding elements: zero)
-      const size_t nA = (size_t)h->N * h->N * h->Kp * 8, nV = (size_t)3 * h->R * h->Kp * 8, nE = (size_t)h->Kp * 4;
+      const size_t nA = (size_t)h->N * h->N * h->Kp * 8, nV = (size_t)3 * h->R * h->Kp * 8, nE = (size_t)op_exp_words(h->p) * h->Kp * 4;
       if ((st = dev_alloc(h, &h->AopX, nA))) return st;
       if ((st = dev_alloc(h, &h->VnX, nV))) return st;
       if ((st = dev_alloc(h, (void **)&h->aopE, nE))) return st;

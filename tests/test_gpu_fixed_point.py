@@ -118,6 +118,60 @@ def test_linear_limiter_matches_fp64_pass(lib, p, e):
     assert rel(_with_handle(cs), _no_alloc(cs)) <= TOL
 
 
+# ... and each element on its own, down to states of 2^-720: none loses its mean or what is left of its slopes
+@pytest.mark.parametrize('e', [-399, -401, -410, -450, -470, -690, -720])
+@pytest.mark.parametrize('p', [1, 2, 3])
+def test_linear_limiter_of_small_states_element_by_element(lib, p, e):
+    from test_zz_no_alloc import _case, _no_alloc, _with_handle
+    cs = _case(1.0 / 9, p, seed=11 + p, jitter=0.2, with_data=True)
+    cs['c'] = np.asfortranarray(np.ldexp(cs['c'], e))
+    cs['data'] = np.asfortranarray(np.ldexp(cs['data'], e))
+    a, b = (np.ldexp(x, -e) for x in (_with_handle(cs), _no_alloc(cs)))
+    assert np.all(np.linalg.norm(a - b, axis=1) <= TOL * np.linalg.norm(b, axis=1))
+
+
+# the range of the matrices, 2^-200 .. 2^400: a velocity scaled by a power of two and the step by its inverse
+@pytest.mark.parametrize('e', [-230, -201, -180, 380, 420])
+@pytest.mark.parametrize('p', [0, 1, 2, 3])
+def test_operator_over_the_velocity_range(lib, p, e):
+    from festung_gb300 import _lib as L
+    from festung_gb300.solver import DeviceSolver
+    coordV, V0T = mesh(9)
+    K, N = len(V0T), (p + 1) * (p + 2) // 2
+    vn = np.repeat(L.grid_build(coordV, V0T)['nuE0T'].sum(axis=2)[:, :, None], p + 1, axis=2)
+    c, out = state(K, N, 6), []
+    for sc in (0, e):
+        s = DeviceSolver(coordV, V0T, p, min(p + 1, 3), precision='fp64', isSlopeLim=False)
+        try:
+            u = np.zeros((K, N), order='F')
+            u[:, 0] = 2.0 ** sc / np.sqrt(2)
+            s.set_velocity(u, u, np.asfortranarray(np.ldexp(vn, sc)))
+            out.append(step(s, c, 1e-3 * 2.0 ** -sc))
+        finally:
+            s.close()
+    assert rel(out[1], out[0]) <= TOL
+
+
+# The time-derivative limiter's sums in fixed point against its FP64 form (the correction rebuilt from the
+# mesh, whose tables differ by rounding; a derivative of order 3 carries 1e-11 of the mean from them)
+@pytest.mark.parametrize('e', [-720, -460, -40, 0, 390, 420])
+@pytest.mark.parametrize('p', [2, 3])
+def test_derivative_limiter_matches_fp64_form(lib, p, e):
+    from festung_gb300 import _lib as L
+    out = []
+    for fly in (0, 1):
+        s = solver(9, p, lim=True)
+        try:
+            s.set_option(L.OPT_TAYLOR_MASS, fly)
+            c = state(2 * 81, (p + 1) * (p + 2) // 2, 5)
+            c[:, 0] += 3.0
+            out.append(step(s, np.ldexp(c, e), 1e-3))
+        finally:
+            s.close()
+    a, b = (np.ldexp(x, -e) for x in out)
+    assert np.all(np.linalg.norm(a - b, axis=1) <= 1e-10 * np.linalg.norm(b, axis=1))
+
+
 # Blocks with more vertices than threads: elements in random order (NO_REORDER keeps it), so 128 of
 # them touch up to 384 vertices.  Minima and maxima do not depend on the order, and an
 # element's arithmetic does not either: bitwise equal to the library's own order.
