@@ -1150,7 +1150,7 @@ __device__ __forceinline__ void stage_op_tile(const Geo<T> g, const T *cin, cons
     __syncthreads();
     if (t == 0) {                                 // static rows before the dependency wait
       stage_expect<T>(bar, NT - (MODE != 2 && first ? N : 0), 1);
-      if constexpr (FXP) {       // digits: 8 bytes each, as the rows they stand for
+      if (FXP && g.AopX) {       // digits: 8 bytes each, as the rows they stand for
         stage_T(smem, rF, (const T *)g.AopX, N * N, Kp, k0, bar);
         stage_T(smem, rV, (const T *)g.VnX, 3 * R, Kp, k0, bar);
       } else {
@@ -1173,7 +1173,7 @@ __device__ __forceinline__ void stage_op_tile(const Geo<T> g, const T *cin, cons
   fx::OpExp<P> ax;
   T src[N];                                       // the source terms at this stage's time
   if constexpr (FXP) {                            // neighbours across inflow edges only
-    if (active) ax.load(g.aopE, Kp, k);
+    if (active && g.aopE) ax.load(g.aopE, Kp, k);
     if (g.rhsM) {
 #pragma unroll
       for (int i = 0; i < N; ++i) src[i] = T(0);
@@ -1185,7 +1185,7 @@ __device__ __forceinline__ void stage_op_tile(const Geo<T> g, const T *cin, cons
     }
 #pragma unroll
     for (int n = 0; n < 3; ++n)
-      if (active && !ax.inflow(n)) nb[n] = -1;
+      if (active && g.aopE && !ax.inflow(n)) nb[n] = -1;
   }
   pdl_wait();
   pdl_trigger();

@@ -71,10 +71,10 @@ struct dgadv_handle {
   void *Aop = nullptr;
   int aopVersion = -1;
   // FP64: digits of Aop, Vn and the linear limiter's correction rows, with their exponents
-  // (dgadv_fixed.cuh)
+  // (dgadv_fixed.cuh); null where they did not fit
   void *AopX = nullptr, *VnX = nullptr, *MTX = nullptr;
   int *aopE = nullptr, *mtE = nullptr;
-  void *rhsM = nullptr;                // FP64: the source terms with hatM^-1 applied
+  void *rhsM = nullptr;                // FP64: the source terms with hatM^-1 applied (null: did not fit)
   // linked stepping (dgadv_link): this handle steps the handles in `linked` together with itself,
   // one launch per stage kernel; a handle in another's list has that handle as linkedTo
   std::vector<dgadv_handle *> linked;
@@ -300,6 +300,7 @@ const PrecOps &ops_of(const dgadv_handle *h);
 
 // Shared host helpers of the C-ABI units (dgadv_solver.cu).
 int dev_alloc(dgadv_handle *h, void **p, size_t bytes);
+void dev_free_from(dgadv_handle *h, size_t mark);   // frees the buffers allocated since h->allocs had `mark`
 int upload(dgadv_handle *h, void *dst, const void *src, size_t bytes);
 int upload_real(dgadv_handle *h, void *dst, const std::vector<double> &src);
 // Volume factors F (2Q x Kp) and edge factors Vn (3R x Kp) of one velocity, internal order.

@@ -899,15 +899,7 @@ struct Solver {
   }
 };
 
-int ensure_state(dgadv_handle *h, int restart) {
-  if (h->impl && h->impl->m >= restart) return DGADV_OK;
-  if (h->impl) {   // a longer restart: the basis is reallocated, the old buffers stay with the handle
-    cudaStreamSynchronize(h->stream);
-    implicit_release(h);
-  }
-  ImplicitState *st = new (std::nothrow) ImplicitState();
-  if (!st) return DGADV_ENOMEM;
-  h->impl = st;
+int allocate_state(dgadv_handle *h, ImplicitState *st, int restart) {
   const size_t rb = ops_of(h).realBytes;
   st->m = restart;
   st->n = (size_t)h->N * h->Kp;
@@ -933,6 +925,24 @@ int ensure_state(dgadv_handle *h, int restart) {
   DG_CUDA(cudaMemsetAsync(st->kst, 0, 4 * vb, h->stream));
   DG_CUDA(cudaStreamSynchronize(h->stream));
   return DGADV_OK;
+}
+
+int ensure_state(dgadv_handle *h, int restart) {
+  if (h->impl && h->impl->m >= restart) return DGADV_OK;
+  if (h->impl) {   // a longer restart: the basis is reallocated, the old buffers stay with the handle
+    cudaStreamSynchronize(h->stream);
+    implicit_release(h);
+  }
+  h->impl = new (std::nothrow) ImplicitState();
+  if (!h->impl) return DGADV_ENOMEM;
+  const size_t mark = h->allocs.size();
+  const int e = allocate_state(h, h->impl, restart);
+  if (e != DGADV_OK) {   // none half made: a later call starts over
+    implicit_release(h);
+    dev_free_from(h, mark);
+    cudaGetLastError();
+  }
+  return e;
 }
 
 template <typename T, int P>

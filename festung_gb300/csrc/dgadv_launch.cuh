@@ -547,6 +547,7 @@ static cudaError_t dispatch_build_element_operator(dgadv_handle *h) {
       case 3: if constexpr ((MASK & 8) != 0) k_build_element_operator<T, 3><<<grid, kBlock, 0, h->stream>>>(g, (T *)h->Aop); break;
     }
     if constexpr (std::is_same_v<T, double>) {
+      if (!h->AopX) return cudaGetLastError();
       auto fix = [&](auto P_) {
         constexpr int P = decltype(P_)::value;
         k_fix_operator<P><<<grid, kBlock, 0, h->stream>>>(h->K, h->Kp, (const double *)h->Aop, (const double *)h->Vn,

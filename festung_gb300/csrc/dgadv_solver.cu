@@ -34,9 +34,36 @@ void dgadv::set_error(const dgadv_handle *h, const char *msg) {
 int dgadv::dev_alloc(dgadv_handle *h, void **p, size_t bytes) {
   if (bytes == 0) bytes = 16;
   cudaError_t e = cudaMalloc(p, bytes);
-  if (e != cudaSuccess) { h->err = std::string("cudaMalloc: ") + cudaGetErrorString(e); return DGADV_ENOMEM; }
+  if (e != cudaSuccess) {
+    *p = nullptr;
+    cudaGetLastError();   // reported here: the thread's next call starts without it
+    h->err = std::string("cudaMalloc: ") + cudaGetErrorString(e);
+    return DGADV_ENOMEM;
+  }
   h->allocs.push_back(*p);
   return DGADV_OK;
+}
+
+// Buffers that work can do without: all of them, zeroed, or none (the pointers stay null).
+static bool alloc_optional(dgadv_handle *h, std::initializer_list<std::pair<void **, size_t>> bufs) {
+  const size_t mark = h->allocs.size();
+  const std::string err = h->err;
+  bool ok = true;
+  for (const auto &b : bufs)
+    ok = ok && dev_alloc(h, b.first, b.second) == DGADV_OK && cudaMemset(*b.first, 0, b.second) == cudaSuccess;
+  if (ok) return true;
+  dgadv::dev_free_from(h, mark);
+  for (const auto &b : bufs) *b.first = nullptr;
+  cudaGetLastError();
+  h->err = err;
+  return false;
+}
+
+void dgadv::dev_free_from(dgadv_handle *h, size_t mark) {
+  while (h->allocs.size() > mark) {
+    cudaFree(h->allocs.back());
+    h->allocs.pop_back();
+  }
 }
 
 int dgadv::upload(dgadv_handle *h, void *dst, const void *src, size_t bytes) {
@@ -367,13 +394,9 @@ static int create_impl(const dgadv_mesh *mesh, const dgadv_params *prm, const st
     }
   }
   if (ops(h).fix_correction && h->limdot && h->limType == DGADV_LIM_LINEAR) {
-    const size_t nQ = (size_t)N * (N - 1) * Kp * 8;
-    if ((st = dev_alloc(h, &h->MTX, nQ))) return st;
-    const size_t nE = (size_t)corr_exp_words(h->p) * Kp * 4;
-    if ((st = dev_alloc(h, (void **)&h->mtE, nE))) return st;
-    DG_CUDA(cudaMemset(h->MTX, 0, nQ));
-    DG_CUDA(cudaMemset(h->mtE, 0, nE));
-    DG_CUDA(ops(h).fix_correction(h));
+    if (alloc_optional(h, {{&h->MTX, (size_t)N * (N - 1) * Kp * 8},
+                           {(void **)&h->mtE, (size_t)corr_exp_words(h->p) * Kp * 4}}))
+      DG_CUDA(ops(h).fix_correction(h));
   }
   DG_CUDA(cudaDeviceSynchronize());
   return DGADV_OK;
@@ -508,9 +531,9 @@ extern "C" int dgadv_set_source_terms(dgadv_handle *h, int32_t nTerms, const int
   if (cDV0T && !h->cDV0T && (st = dev_alloc(h, &h->cDV0T, 4 * (size_t)3 * Kp * w))) return st;
   if ((st = upload_real(h, h->rhs, r))) return st;
   if (h->prec == DGADV_FP64 && !(h->flags & DGADV_FLAG_IMPLICIT)) {   // with hatM^-1 applied
-    if (!h->rhsM && (st = dev_alloc(h, &h->rhsM, 4 * (size_t)N * Kp * w))) return st;
-    std::vector<double> rm(r.size(), 0.0);
-    for (int m = 0; m < nTerms; ++m)
+    if (!h->rhsM) alloc_optional(h, {{&h->rhsM, 4 * (size_t)N * Kp * w}});   // else the quadrature form
+    std::vector<double> rm(h->rhsM ? r.size() : 0, 0.0);
+    for (int m = 0; m < nTerms && h->rhsM; ++m)
       for (int i = 0; i < N; ++i)
         for (int j = 0; j < N; ++j) {
           const double a = h->tables.hatMinv[i * N + j];
@@ -518,7 +541,7 @@ extern "C" int dgadv_set_source_terms(dgadv_handle *h, int32_t nTerms, const int
           double *dst = &rm[((size_t)m * N + i) * Kp];
           for (int k = 0; k < K; ++k) dst[k] += a * src[k];
         }
-    if ((st = upload_real(h, h->rhsM, rm))) return st;
+    if (h->rhsM && (st = upload_real(h, h->rhsM, rm))) return st;
   }
   if (cDV0T && (st = upload_real(h, h->cDV0T, d))) return st;
   if (!cDV0T && h->cDV0T) DG_CUDA(cudaMemset(h->cDV0T, 0, 4 * (size_t)3 * Kp * w));
@@ -764,15 +787,9 @@ int dgadv::refresh_element_operator(dgadv_handle *h) {
     int st;
     if ((st = dev_alloc(h, &h->Aop, (size_t)h->N * h->N * h->Kp * o.realBytes))) return st;
     DG_CUDA(cudaMemset(h->Aop, 0, (size_t)h->N * h->N * h->Kp * o.realBytes));
-    if (h->prec == DGADV_FP64) {   // its digits (padding elements: zero)
-      const size_t nA = (size_t)h->N * h->N * h->Kp * 8, nV = (size_t)3 * h->R * h->Kp * 8, nE = (size_t)op_exp_words(h->p) * h->Kp * 4;
-      if ((st = dev_alloc(h, &h->AopX, nA))) return st;
-      if ((st = dev_alloc(h, &h->VnX, nV))) return st;
-      if ((st = dev_alloc(h, (void **)&h->aopE, nE))) return st;
-      DG_CUDA(cudaMemset(h->AopX, 0, nA));
-      DG_CUDA(cudaMemset(h->VnX, 0, nV));
-      DG_CUDA(cudaMemset(h->aopE, 0, nE));
-    }
+    if (h->prec == DGADV_FP64)   // its digits, where there is room: without them the sums run in FP64
+      alloc_optional(h, {{&h->AopX, (size_t)h->N * h->N * h->Kp * 8}, {&h->VnX, (size_t)3 * h->R * h->Kp * 8},
+                         {(void **)&h->aopE, (size_t)op_exp_words(h->p) * h->Kp * 4}});
   }
   DG_CUDA(o.build_element_operator(h));
   // captured steps keep their kernels: they are recaptured once the operator comes into use

@@ -102,12 +102,15 @@ extern "C" int dgadv_transport_init(dgadv_handle *h, int32_t nSpecies, const dou
     TransportState *n = new (std::nothrow) TransportState();
     if (!n) return DGADV_ENOMEM;
     h->trans = n;
+    const size_t mark = h->allocs.size();
     if ((e = dev_alloc(h, &n->cH, nSpecies * bytes)) || (e = dev_alloc(h, &n->cHs, nSpecies * bytes)) ||
         (e = dev_alloc(h, &n->conc, nSpecies * bytes)) || (e = dev_alloc(h, &n->work, nSpecies * bytes)) ||
         (e = dev_alloc(h, (void **)&n->mask, nSpecies * Kp)) || (e = dev_alloc(h, &n->hQ, Q * Kp * o.realBytes)) ||
         (e = dev_alloc(h, &n->vkeys, 3 * nSpecies * nKeys * o.keyBytes)) ||
         (e = dev_alloc(h, (void **)&n->slots, 3 * nSpecies * nSlots * 8))) {
       transport_release(h);
+      dev_free_from(h, mark);
+      cudaGetLastError();
       return e;
     }
     n->capacity = nSpecies;
