@@ -123,11 +123,13 @@ static cudaError_t launch_linked_step(dgadv_handle **hs, int n, double /*t0: no 
   size_t vt = 0;                                        // the longest vertex table among the parts
   for (int i = 0; i < n; ++i) vt = std::max(vt, vt_bytes<T>(hs[i], 1));
   const size_t smemOp = link_smem<T, MASK>(0) + vt, smemLd = link_smem<T, MASK>(1) + 2 * vt, smemLm = vt;
-  cudaError_t e = cudaFuncSetAttribute((const void *)k_link_op<T, MASK>,
-                                       cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smemOp);
+  // opted in for the longest tables any handle can have: one size for every group, as groups on other
+  // threads launch the same kernels
+  cudaError_t e = cudaFuncSetAttribute((const void *)k_link_op<T, MASK>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                       (int)(link_smem<T, MASK>(0) + vt_most<T, 1>(1)));
   if (e == cudaSuccess)
     e = cudaFuncSetAttribute((const void *)k_link_limdot<T, MASK>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)smemLd);
+                             (int)(link_smem<T, MASK>(1) + vt_most<T, 1>(2)));
   if (e != cudaSuccess) return e;
   const int eb = h0->opBlock;                           // the operator's elements per block
   int S[kMaxLinked];
