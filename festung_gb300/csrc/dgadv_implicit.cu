@@ -175,12 +175,14 @@ __global__ void __launch_bounds__(kRows * IDims<P>::N) k_impl_op(const ImplArgs<
 
 // Inverse of each element's diagonal block of y = ca x + cb cDot(x) (volume term and the
 // element's own outflow; the neighbours' inflow is off-diagonal), by Gauss-Jordan elimination
-// with partial pivoting in FP64.  A block with a vanishing pivot is replaced by the identity and
-// *singular set.  Aloc receives cDot's local part itself.
+// with partial pivoting in FP64.  A block that is singular to the stored type's rounding (a pivot below
+// N eps of its largest entry) is replaced by the identity; *inexact is set then, and where the block
+// times the stored inverse is off the identity by more than sqrt(eps).  Aloc receives cDot's
+// local part itself.
 template <typename T, int P>
 __global__ void __launch_bounds__(kImplBlock) k_impl_block(const ImplArgs<T> a, double ca, double cb,
                                                            T *__restrict__ Pinv, T *__restrict__ Aloc,
-                                                           int *__restrict__ singular) {
+                                                           int *__restrict__ inexact) {
   constexpr int N = IDims<P>::N, Q = IDims<P>::Q, R = IDims<P>::R;
   const int k = blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= a.K) return;
@@ -212,7 +214,8 @@ __global__ void __launch_bounds__(kImplBlock) k_impl_block(const ImplArgs<T> a, 
       }
     }
   }
-  double A[N][2 * N];
+  constexpr double eps = sizeof(T) == 4 ? 0x1p-24 : 0x1p-53, rootEps = sizeof(T) == 4 ? 0x1p-12 : 0x1p-26;
+  double A[N][2 * N], most = 0.0;
   for (int i = 0; i < N; ++i) {
     for (int j = 0; j < N; ++j) {
       double s = 0.0;
@@ -220,6 +223,7 @@ __global__ void __launch_bounds__(kImplBlock) k_impl_block(const ImplArgs<T> a, 
       Aloc[(size_t)(i * N + j) * Kp + k] = T(s);
       A[i][j] = (i == j ? ca : 0.0) + cb * s;
       A[i][N + j] = i == j ? 1.0 : 0.0;
+      most = fmax(most, fabs(A[i][j]));
     }
   }
   bool ok = true;
@@ -227,7 +231,7 @@ __global__ void __launch_bounds__(kImplBlock) k_impl_block(const ImplArgs<T> a, 
     int piv = col;
     for (int r = col + 1; r < N; ++r)
       if (fabs(A[r][col]) > fabs(A[piv][col])) piv = r;
-    if (!(fabs(A[piv][col]) > 1e-300)) { ok = false; break; }
+    if (!(fabs(A[piv][col]) > N * eps * most)) { ok = false; break; }
     if (piv != col)
       for (int j = 0; j < 2 * N; ++j) { const double t = A[col][j]; A[col][j] = A[piv][j]; A[piv][j] = t; }
     const double inv = 1.0 / A[col][col];
@@ -239,7 +243,16 @@ __global__ void __launch_bounds__(kImplBlock) k_impl_block(const ImplArgs<T> a, 
         for (int j = 0; j < 2 * N; ++j) A[r][j] -= f * A[col][j];
     }
   }
-  if (!ok) *singular = 1;
+  double off = 0.0;             // of the block, as it is applied, times the inverse, as it is stored
+  for (int i = 0; i < N; ++i)
+    for (int j = 0; j < N; ++j) {
+      double s = i == j ? -1.0 : 0.0;
+      for (int l = 0; l < N; ++l)
+        s += ((i == l ? ca : 0.0) + cb * (double)Aloc[(size_t)(i * N + l) * Kp + k]) * (double)T(A[l][N + j]);
+      off = fmax(off, fabs(s));
+      ok = ok && isfinite(s);
+    }
+  if (!ok || off > rootEps) *inexact = 1;
   for (int i = 0; i < N; ++i)
     for (int j = 0; j < N; ++j) Pinv[(i * N + j) * Kp + k] = T(ok ? A[i][N + j] : (i == j ? 1.0 : 0.0));
 }
@@ -394,8 +407,8 @@ struct GmresDense {
 // elements, p = 2; now 45 us):
 //   k_arn_apply   w = A P^-1 v_j; h1 = V^T w.  z = P^-1 v_j comes from the step before.  P inverts the
 //                 element's own block of A, so the local part of A z is v_j itself and only the
-//                 neighbours' inflow is left (IDENT; a mesh with a singular block, whose P is the
-//                 identity there, applies the whole operator)
+//                 neighbours' inflow is left (IDENT; a mesh with a block whose stored inverse is off, or
+//                 singular with the identity in its place, applies the whole operator)
 //   k_arn_first   w -= V h1; h2 = V^T w and |w|^2        (classical Gram-Schmidt, second pass)
 //   k_arn_second  w -= V h2; v_{j+1} = w / |w|, with |w|^2 after the pass from |w|^2 - |h2|^2 (h2 is at
 //                 rounding level: no cancellation); z = P^-1 v_{j+1}; column j of the Hessenberg matrix and
@@ -663,7 +676,7 @@ struct ImplicitState {
   double pinvA = 0.0, pinvB = 0.0;
   int pinvVersion = -1;           // velocity version the blocks were built for
   void *Aloc = nullptr;           // N^2 x Kp: cDot's local part
-  int *singular = nullptr;        // a diagonal block was singular
+  int *inexact = nullptr;         // a diagonal block was singular, or its stored inverse is off
   bool ident = false;             // ... none was: P^-1 inverts every diagonal block
   int blocks = 0;                 // the element kernels' blocks
   double *partial = nullptr;      // (m + 2) x blocks
@@ -753,13 +766,13 @@ struct Solver {
   // coefficients changed.
   int build_prec(double ca, double cb) {
     if (st->pinvVersion == h->velVersion && st->pinvA == ca && st->pinvB == cb) return DGADV_OK;
-    int sing = 0;
-    DG_CUDA(cudaMemsetAsync(st->singular, 0, sizeof(int), h->stream));
-    k_impl_block<T, P><<<st->blocks, kRows, 0, h->stream>>>(args, ca, cb, (T *)st->Pinv, (T *)st->Aloc, st->singular);
-    DG_CUDA(cudaMemcpyAsync(&sing, st->singular, sizeof(int), cudaMemcpyDeviceToHost, h->stream));
+    int inexact = 0;
+    DG_CUDA(cudaMemsetAsync(st->inexact, 0, sizeof(int), h->stream));
+    k_impl_block<T, P><<<st->blocks, kRows, 0, h->stream>>>(args, ca, cb, (T *)st->Pinv, (T *)st->Aloc, st->inexact);
+    DG_CUDA(cudaMemcpyAsync(&inexact, st->inexact, sizeof(int), cudaMemcpyDeviceToHost, h->stream));
     DG_CUDA(cudaStreamSynchronize(h->stream));
-    if (st->ident != (sing == 0)) st->graphA = st->graphB = 0.0;   // the steps' graphs hold the other kernel
-    st->ident = sing == 0;
+    if (st->ident != (inexact == 0)) st->graphA = st->graphB = 0.0;   // the steps' graphs hold the other kernel
+    st->ident = inexact == 0;
     st->pinvA = ca; st->pinvB = cb; st->pinvVersion = h->velVersion;
     return DGADV_OK;
   }
@@ -915,7 +928,7 @@ int allocate_state(dgadv_handle *h, ImplicitState *st, int restart) {
   st->blocks = (h->K + kRows - 1) / kRows;
   if ((e = dev_alloc(h, (void **)&st->partial, (size_t)(restart + 2) * st->blocks * 8))) return e;
   if ((e = dev_alloc(h, (void **)&st->ticket, 16))) return e;
-  if ((e = dev_alloc(h, (void **)&st->singular, 16))) return e;
+  if ((e = dev_alloc(h, (void **)&st->inexact, 16))) return e;
   if ((e = dev_alloc(h, (void **)&st->dres, (size_t)(2 * restart + 3) * 8))) return e;
   DG_CUDA(cudaMemsetAsync(st->ticket, 0, 16, h->stream));
   if ((e = dev_alloc(h, (void **)&st->dense, ((size_t)(restart + 1) * restart + 4 * (size_t)restart + 8) * 8))) return e;
