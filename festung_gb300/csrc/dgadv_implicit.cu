@@ -259,8 +259,13 @@ __global__ void __launch_bounds__(kImplBlock) k_impl_block(const ImplArgs<T> a, 
 
 // ---- vector kernels over n = N Kp values ------------------------------------------------------
 
-// A sum over the grid in a fixed order: every block adds its threads' shares, the block that
-// arrives last adds the blocks' (in block order, whichever block it is).
+// A sum over the grid in a fixed order: every block adds its threads' shares, group after group of 32
+// elements, the block that arrives last adds the blocks' (in block order, whichever block it is).
+// kSumBlocks blocks at most, as many as the SMs hold at a time, so that this last addition stays short
+// beside the kernel: with a block per group, one block was left K / 32 shares of every basis vector
+// (524288 triangles, an Arnoldi step in FP64: p = 1 905 us so and 397 now, p = 2 1361 and 768; 32768
+// triangles, 1024 groups either way, 78 and 83 us).
+constexpr int kSumBlocks = 8 * 152;
 struct GridSums {
   double *partial;          // vector v, block b at v * gridDim.x + b
   unsigned int *ticket;     // blocks that have stored their shares (0 between launches)
@@ -296,9 +301,11 @@ template <int n> __device__ __forceinline__ void warp_sums(double x[n]) {
 #pragma unroll
   for (int q = 0; q < n; ++q) x[q] = fx::to_double_int(v[q], max(E[q], 223) - 1022 - 57);
 }
-// The threads' shares x[0 .. n) of vectors v0 ...: added over the block into partial.
+// The threads' shares x[0 .. n) of vectors v0 ...: added over the block into tot (the block's sums, set by its
+// first group).
+constexpr int kMaxSums = 258;
 template <int N>
-__device__ __forceinline__ void store_shares(const GridSums &gs, int v0, int n, double x[kVecs]) {
+__device__ __forceinline__ void add_shares(double *tot, bool first, int v0, int n, double x[kVecs]) {
   __shared__ double sh[N][kVecs];
   __syncthreads();                            // the shares before are read
   if (n <= 2) warp_sums<2>(x);                // the values beyond n are zero
@@ -312,13 +319,15 @@ __device__ __forceinline__ void store_shares(const GridSums &gs, int v0, int n, 
     double s = 0.0;
 #pragma unroll
     for (int i = 0; i < N; ++i) s += sh[i][threadIdx.x];
-    gs.partial[(size_t)(v0 + threadIdx.x) * gridDim.x + blockIdx.x] = s;
+    tot[v0 + threadIdx.x] = first ? s : tot[v0 + threadIdx.x] + s;   // always this thread's
   }
 }
 // After the shares of nv vectors: the last block writes their sums.
 template <int N>
-__device__ __forceinline__ void finish_sums(const GridSums &gs, int nv) {
+__device__ __forceinline__ void finish_sums(const GridSums &gs, const double *tot, int nv) {
   __shared__ bool last;
+  __syncthreads();
+  for (int v = threadIdx.y * 32 + threadIdx.x; v < nv; v += 32 * N) gs.partial[(size_t)v * gridDim.x + blockIdx.x] = tot[v];
   __threadfence();
   __syncthreads();
   if (threadIdx.x == 0 && threadIdx.y == 0) last = atomicAdd(gs.ticket, 1u) == gridDim.x - 1;
@@ -343,14 +352,14 @@ __device__ __forceinline__ void finish_sums(const GridSums &gs, int nv) {
 }
 // The shares of <V_v, y> for v < nv, at = row Kp + k the thread's place (inactive: y = 0, at within V).
 template <typename T, int N>
-__device__ __forceinline__ void share_products(const GridSums &gs, const T *V, size_t n, size_t at, int nv, double y) {
+__device__ __forceinline__ void share_products(double *tot, bool first, const T *V, size_t n, size_t at, int nv, double y) {
   for (int v0 = 0; v0 < nv; v0 += kVecs) {
     double s[kVecs];
 #pragma unroll
     for (int q = 0; q < kVecs; ++q) s[q] = v0 + q < nv ? (double)V[(size_t)(v0 + q) * n + at] : 0.0;
 #pragma unroll
     for (int q = 0; q < kVecs; ++q) s[q] *= y;
-    store_shares<N>(gs, v0, min(kVecs, nv - v0), s);
+    add_shares<N>(tot, first, v0, min(kVecs, nv - v0), s);
   }
 }
 // y + sgn sum_{v < nv} h_v V_v at the thread's place
@@ -419,40 +428,45 @@ k_arn_apply(const ImplArgs<T> a, const T *__restrict__ V, size_t n, int j, const
             double ca, double cb, const GridSums gs) {
   constexpr int N = IDims<P>::N;
   __shared__ T fl[3 * IDims<P>::R][kRows];
-  const int k = blockIdx.x * kRows + threadIdx.x;
-  const bool act = k < a.K;
-  const size_t at = (size_t)threadIdx.y * a.Kp + (act ? k : 0);
-  EdgePoints<T, P> ep;
-  ep.load(a, k, act);
-  const T s = cdot_row<T, P, !IDENT>(a, ep, z, k, act, fl);
-  T y = T(0);
-  if (act) {
-    y = (IDENT ? V[(size_t)j * n + at] : T(ca) * z[at]) + T(cb) * s;
-    w[at] = y;
+  __shared__ double tot[kMaxSums];
+  for (int grp = blockIdx.x; grp * kRows < a.K; grp += gridDim.x) {
+    const int k = grp * kRows + threadIdx.x;
+    const bool act = k < a.K;
+    const size_t at = (size_t)threadIdx.y * a.Kp + (act ? k : 0);
+    EdgePoints<T, P> ep;
+    ep.load(a, k, act);
+    const T s = cdot_row<T, P, !IDENT>(a, ep, z, k, act, fl);
+    T y = T(0);
+    if (act) {
+      y = (IDENT ? V[(size_t)j * n + at] : T(ca) * z[at]) + T(cb) * s;
+      w[at] = y;
+    }
+    share_products<T, N>(tot, grp == (int)blockIdx.x, V, n, at, j + 1, (double)y);
   }
-  share_products<T, N>(gs, V, n, at, j + 1, (double)y);
-  finish_sums<N>(gs, j + 1);
+  finish_sums<N>(gs, tot, j + 1);
 }
 
 template <typename T, int N>
 __global__ void __launch_bounds__(kRows * N) k_arn_first(int K, int Kp, const T *V, size_t n, int j, T *w,
                                                          const double *h1, const GridSums gs) {
-  __shared__ double sh[257];
+  __shared__ double sh[257], tot[kMaxSums];
   for (int v = threadIdx.y * 32 + threadIdx.x; v <= j; v += 32 * N) sh[v] = h1[v];
-  const int k = blockIdx.x * kRows + threadIdx.x;
-  const bool act = k < K;
-  const size_t at = (size_t)threadIdx.y * Kp + (act ? k : 0);
-  double y = act ? (double)w[at] : 0.0;
   __syncthreads();
-  if (act) {
-    const T t = T(add_vectors(V, n, at, j + 1, sh, -1.0, y));
-    w[at] = t;
-    y = (double)t;
+  for (int grp = blockIdx.x; grp * kRows < K; grp += gridDim.x) {
+    const int k = grp * kRows + threadIdx.x;
+    const bool act = k < K, first = grp == (int)blockIdx.x;
+    const size_t at = (size_t)threadIdx.y * Kp + (act ? k : 0);
+    double y = act ? (double)w[at] : 0.0;
+    if (act) {
+      const T t = T(add_vectors(V, n, at, j + 1, sh, -1.0, y));
+      w[at] = t;
+      y = (double)t;
+    }
+    share_products<T, N>(tot, first, V, n, at, j + 1, y);
+    double s[kVecs] = {y * y};
+    add_shares<N>(tot, first, j + 1, 1, s);
   }
-  share_products<T, N>(gs, V, n, at, j + 1, y);
-  double s[kVecs] = {y * y};
-  store_shares<N>(gs, j + 1, 1, s);
-  finish_sums<N>(gs, j + 2);
+  finish_sums<N>(gs, tot, j + 2);
 }
 
 // Column j: h1 + h2, the earlier rotations, a new one, the residual estimate.  One warp; the chain of
@@ -545,21 +559,24 @@ k_impl_residual(const ImplArgs<T> a, const T *__restrict__ b, const T *__restric
                 double cb, const GridSums gs) {
   constexpr int N = IDims<P>::N;
   __shared__ T fl[3 * IDims<P>::R][kRows];
-  const int k = blockIdx.x * kRows + threadIdx.x;
-  const bool act = k < a.K;
-  const size_t at = (size_t)threadIdx.y * a.Kp + (act ? k : 0);
-  EdgePoints<T, P> ep;
-  ep.load(a, k, act);
-  const T s = cdot_row<T, P, true>(a, ep, x, k, act, fl);
-  double q[kVecs] = {0.0};
-  if (act) {
-    const T bi = b[at], y = T(ca) * x[at] + T(cb) * s, ri = T((double)bi - (double)y);
-    r[at] = ri;
-    q[0] = (double)ri * (double)ri;
-    q[1] = (double)bi * (double)bi;
+  __shared__ double tot[2];
+  for (int grp = blockIdx.x; grp * kRows < a.K; grp += gridDim.x) {
+    const int k = grp * kRows + threadIdx.x;
+    const bool act = k < a.K;
+    const size_t at = (size_t)threadIdx.y * a.Kp + (act ? k : 0);
+    EdgePoints<T, P> ep;
+    ep.load(a, k, act);
+    const T s = cdot_row<T, P, true>(a, ep, x, k, act, fl);
+    double q[kVecs] = {0.0};
+    if (act) {
+      const T bi = b[at], y = T(ca) * x[at] + T(cb) * s, ri = T((double)bi - (double)y);
+      r[at] = ri;
+      q[0] = (double)ri * (double)ri;
+      q[1] = (double)bi * (double)bi;
+    }
+    add_shares<N>(tot, grp == (int)blockIdx.x, 0, 2, q);
   }
-  store_shares<N>(gs, 0, 2, q);
-  finish_sums<N>(gs, 2);
+  finish_sums<N>(gs, tot, 2);
 }
 
 // v_0 = r / |r|, z = P^-1 v_0, and the dense part of a new cycle.
@@ -678,8 +695,9 @@ struct ImplicitState {
   void *Aloc = nullptr;           // N^2 x Kp: cDot's local part
   int *inexact = nullptr;         // a diagonal block was singular, or its stored inverse is off
   bool ident = false;             // ... none was: P^-1 inverts every diagonal block
-  int blocks = 0;                 // the element kernels' blocks
-  double *partial = nullptr;      // (m + 2) x blocks
+  int blocks = 0;                 // the element kernels' blocks: one per group of 32
+  int sumBlocks = 0;              // ... of those that add over the grid
+  double *partial = nullptr;      // (m + 2) x sumBlocks
   unsigned int *ticket = nullptr;
   double *dres = nullptr;         // h1 (m + 1), h2 and |w|^2 (m + 2)
   double *dense = nullptr;        // H ((m + 1) x m), cs, sn, g, y, status
@@ -781,13 +799,13 @@ struct Solver {
   // Arnoldi step j: w = A P^-1 v_j, orthogonalised against v_0..v_j (classical Gram-Schmidt,
   // twice), v_{j+1} = w / |w|, z = P^-1 v_{j+1}, and the dense update of column j.
   void arnoldi_enqueue(int j, double ca, double cb, const GmresDense &d) {
-    const int m = st->m, nb = st->blocks;
+    const int m = st->m, nb = st->blocks, ns = st->sumBlocks;
     const dim3 nt(kRows, N);
     T *w = vec(st->w), *z = vec(st->z), *V = basis(0);
     double *h1 = st->dres, *h2 = st->dres + (m + 1);
-    if (st->ident) k_arn_apply<T, P, true><<<nb, nt, 0, h->stream>>>(args, V, n, j, z, w, ca, cb, sums(h1));
-    else k_arn_apply<T, P, false><<<nb, nt, 0, h->stream>>>(args, V, n, j, z, w, ca, cb, sums(h1));
-    k_arn_first<T, N><<<nb, nt, 0, h->stream>>>(h->K, h->Kp, V, n, j, w, h1, sums(h2));
+    if (st->ident) k_arn_apply<T, P, true><<<ns, nt, 0, h->stream>>>(args, V, n, j, z, w, ca, cb, sums(h1));
+    else k_arn_apply<T, P, false><<<ns, nt, 0, h->stream>>>(args, V, n, j, z, w, ca, cb, sums(h1));
+    k_arn_first<T, N><<<ns, nt, 0, h->stream>>>(h->K, h->Kp, V, n, j, w, h1, sums(h2));
     k_arn_second<T, N><<<nb + 1, nt, 0, h->stream>>>(h->K, h->Kp, V, n, j, w, (const T *)st->Pinv, z, h1, h2, d, m);
   }
   // Steps j .. j + cnt - 1: kCheck of them, between two looks at the residual, as one CUDA graph captured
@@ -836,7 +854,7 @@ struct Solver {
     d.status = d.y + m;
     int used = 0;
     for (;;) {
-      k_impl_residual<T, P><<<nb, nt, 0, h->stream>>>(args, b, x, r, ca, cb, sums(st->dres));
+      k_impl_residual<T, P><<<st->sumBlocks, nt, 0, h->stream>>>(args, b, x, r, ca, cb, sums(st->dres));
       cudaMemcpyAsync(st->hres, st->dres, 2 * sizeof(double), cudaMemcpyDeviceToHost, h->stream);
       if (cudaStreamSynchronize(h->stream) != cudaSuccess) return DGADV_ECUDA;
       const double bnorm = std::sqrt(st->hres[1]);
@@ -926,7 +944,8 @@ int allocate_state(dgadv_handle *h, ImplicitState *st, int restart) {
   if ((e = dev_alloc(h, &st->Pinv, (size_t)h->N * h->N * h->Kp * rb))) return e;
   if ((e = dev_alloc(h, &st->Aloc, (size_t)h->N * h->N * h->Kp * rb))) return e;
   st->blocks = (h->K + kRows - 1) / kRows;
-  if ((e = dev_alloc(h, (void **)&st->partial, (size_t)(restart + 2) * st->blocks * 8))) return e;
+  st->sumBlocks = std::min(st->blocks, kSumBlocks);
+  if ((e = dev_alloc(h, (void **)&st->partial, (size_t)(restart + 2) * st->sumBlocks * 8))) return e;
   if ((e = dev_alloc(h, (void **)&st->ticket, 16))) return e;
   if ((e = dev_alloc(h, (void **)&st->inexact, 16))) return e;
   if ((e = dev_alloc(h, (void **)&st->dres, (size_t)(2 * restart + 3) * 8))) return e;
