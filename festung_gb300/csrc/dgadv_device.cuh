@@ -433,8 +433,8 @@ __device__ __forceinline__ bool nan_(const df32 &x) { return x.hi != x.hi || x.l
 // the block's empty key table at vtOff (a block barrier has to follow before scatter_quantities).
 // 32-bit keys only: a 64-bit minimum in shared memory is a compare-and-swap loop (measured: FP64
 // operator on 2048 triangles 7.2 -> 9.0 us).
-template <typename T> __device__ __forceinline__ bool vt_on() {
-  return sizeof(typename KeyOf<T>::type) == 4 && blockDim.x == kBlock;
+template <typename T> __device__ __forceinline__ bool vt_on(const Geo<T> &g, int nc) {
+  return sizeof(typename KeyOf<T>::type) == 4 && blockDim.x == kBlock && use_block_tables(nc, g.vtMax);
 }
 // The block's vertex list: its bounds and this thread's vertex, read before the dependency wait.
 struct VtList {
@@ -814,6 +814,31 @@ __device__ __forceinline__ void patch_minmax(const LimIn<T> &, const PatchView<T
     mx[n] = fmax(kv.pv[(2 * s + 1) * kv.stride + kv.l[n]], valD[n]);
   }
 }
+// The same from the element's own keys, where the block has no table (use_block_tables).
+template <typename T> struct PatchKeys {
+  int Vp, v[3];     // vertex ids
+};
+template <typename T, int NQ>
+__device__ __forceinline__ void patch_minmax(const LimIn<T> &li, const PatchKeys<T> &kv, const T *sh, int s,
+                                             const T valD[3], T mn[3], T mx[3]) {
+#pragma unroll
+  for (int n = 0; n < 3; ++n) {
+    T a = vkey_inv<T>(li.vkeys[(size_t)(2 * s) * kv.Vp + kv.v[n]]);
+    T c = vkey_inv<T>(li.vkeys[(size_t)(2 * s + 1) * kv.Vp + kv.v[n]]);
+    if (li.shift) { a = (a - sh[2 * s + 1]) + sh[2 * s + 1]; c = (c + sh[2 * s]) - sh[2 * s]; }
+    mn[n] = fmin(a, valD[n]);
+    mx[n] = fmax(c, valD[n]);
+  }
+}
+template <typename T>
+__device__ __forceinline__ PatchView<T> patch_view(const Geo<T> &g, int vtIn, const int vid[3], std::true_type) {
+  extern __shared__ __align__(128) unsigned char smem[];
+  return PatchView<T>{(const T *)(smem + vtIn), g.vtMax, {vid[0], vid[1], vid[2]}};
+}
+template <typename T>
+__device__ __forceinline__ PatchKeys<T> patch_view(const Geo<T> &g, int, const int vid[3], std::false_type) {
+  return PatchKeys<T>{g.Vp, {vid[0], vid[1], vid[2]}};
+}
 // The extremes alone (no boundary data).
 template <typename T>
 __device__ __forceinline__ void patch_extremes(const PatchView<T> &kv, T mn[3], T mx[3]) {
@@ -1142,7 +1167,7 @@ __device__ __forceinline__ void stage_op_tile(const Geo<T> g, const T *cin, cons
   const bool staged = k0 < g.K;                   // blocks beyond the elements only reset keys
   const bool first = sc.omega == 0.0;             // c^n has no part in this stage: not read
   constexpr int rC = 0, rC0 = N, rF = (MODE != 2) ? 2 * N : N, rV = rF + (EOP ? N * N : 2 * Q), rB = rV + 3 * R;
-  const bool vt = MODE != 0 && vt_on<T>();
+  const bool vt = MODE != 0 && vt_on<T>(g, lo.nc);
   const int vtOff = vt ? (int)StageRows<T, P>::bytes(NT, 1) : -1;
   if (staged) {
     if (t == 0) { mbar_init(bar, 1); mbar_fence_init(); }
@@ -1611,7 +1636,7 @@ template <> struct LimDotBlocks<float, 2> { static constexpr int value = 5; };
 template <typename T> struct LimBlocks { static constexpr int value = 1; };
 template <> struct LimBlocks<float> { static constexpr int value = 5; };
 
-template <typename T, int P, int LT>
+template <typename T, int P, int LT, bool TAB>
 __global__ void __launch_bounds__(kBlock, LimDotBlocks<T, LT>::value)
 k_limit_dot(const Geo<T> g, const T *cin, const T *c0, const T *tbuf, T *tout,
             const LimIn<T> li, const LimOut<T> lo, const StageScalars sc) {
@@ -1626,7 +1651,7 @@ k_limit_dot(const Geo<T> g, const T *cin, const T *c0, const T *tbuf, T *tout,
   const int Kp = g.Kp;
   const bool staged = k0 < g.K;
   constexpr int rT = 0, rB = N, rC0 = N + 4, rC = rC0 + N;
-  const int vtIn = (int)StageRows<T, P>::bytes(NT, 1), vtOff = vt_on<T>() ? vtIn + 2 * lo.nc * g.vtMax * (int)sizeof(T) : -1;
+  const int vtIn = (int)StageRows<T, P>::bytes(NT, 1), vtOff = TAB && vt_on<T>(g, lo.nc) ? vtIn + 2 * lo.nc * g.vtMax * (int)sizeof(T) : -1;
   if (staged) {
     if (t == 0) { mbar_init(bar, 1); mbar_fence_init(); }
     if (vtOff >= 0) vt_reset(g, lo.nc, vtOff);
@@ -1639,9 +1664,9 @@ k_limit_dot(const Geo<T> g, const T *cin, const T *c0, const T *tbuf, T *tout,
   }
   const bool active = k < g.K;
   int vid[3] = {0, 0, 0};
-  if (active) load_vertices(g, k, true, vid);
+  if (active) load_vertices(g, k, TAB, vid);
   VtList vl{0, 0, 0};
-  if (staged) vl = vt_list(g, blockIdx.x);
+  if (TAB && staged) vl = vt_list(g, blockIdx.x);
   pdl_wait();
   pdl_trigger();
   reset_next<T>(g, lo, k);
@@ -1651,8 +1676,12 @@ k_limit_dot(const Geo<T> g, const T *cin, const T *c0, const T *tbuf, T *tout,
     stage_T(smem, rC0, c0, N, Kp, k0, bar);
     stage_T(smem, rC, cin, N, Kp, k0, bar);
   }
-  const PatchView<T> pv{(const T *)(smem + vtIn), g.vtMax, {vid[0], vid[1], vid[2]}};
-  load_patch<T, NQ>(g, li, blockIdx.x, vl, sh, vtIn);
+  const auto pv = patch_view<T>(g, vtIn, vid, std::bool_constant<TAB>());
+  if (TAB) load_patch<T, NQ>(g, li, blockIdx.x, vl, sh, vtIn);
+  else {
+    if (li.shift) load_shifts<T>(li.slots + slot_base(g, li.nc), li.nc, sh);
+    __syncthreads();
+  }
   const bool ok = mbar_wait_bounded(bar, sc.flag);
   int gid[3] = {0, 0, 0};   // vertex ids of the direct atomics (64-bit keys)
   if (active && vtOff < 0) load_vertices(g, k, false, gid);
@@ -1734,7 +1763,7 @@ k_limit_dot(const Geo<T> g, const T *cin, const T *c0, const T *tbuf, T *tout,
 
 // Solution limiter: limited Taylor coefficients back to the modal basis
 // (core/applySlopeLimiterDisc.m:77-86).
-template <typename T, int P, int LT>
+template <typename T, int P, int LT, bool TAB>
 __global__ void __launch_bounds__(kBlock, LimBlocks<T>::value)
 k_limit(const Geo<T> g, const T *tbuf, T *__restrict__ out, const LimIn<T> li,
         const StageScalars sc) {
@@ -1756,13 +1785,18 @@ k_limit(const Geo<T> g, const T *tbuf, T *__restrict__ out, const LimIn<T> li,
   const bool active = k < g.K;
   int vid[3] = {0, 0, 0};
   const int vtIn = (int)StageRows<T, P>::bytes(NT, 1);
-  if (active) load_vertices(g, k, true, vid);
-  const VtList vl = vt_list(g, blockIdx.x);
+  if (active) load_vertices(g, k, TAB, vid);
+  VtList vl{0, 0, 0};
+  if (TAB) vl = vt_list(g, blockIdx.x);
   pdl_wait();
   pdl_trigger();
   if (t == 0) stage_T(smem, 0, tbuf, N, Kp, k0, bar);
-  const PatchView<T> pv{(const T *)(smem + vtIn), g.vtMax, {vid[0], vid[1], vid[2]}};
-  load_patch<T, NQ>(g, li, blockIdx.x, vl, sh, vtIn);
+  const auto pv = patch_view<T>(g, vtIn, vid, std::bool_constant<TAB>());
+  if (TAB) load_patch<T, NQ>(g, li, blockIdx.x, vl, sh, vtIn);
+  else {
+    if (li.shift) load_shifts<T>(li.slots + slot_base(g, li.nc), li.nc, sh);
+    __syncthreads();
+  }
   T data[3] = {T(0), T(0), T(0)};
   if (g.cDV0T && active) {
     for (int m = 0; m < g.nTerms; ++m) {
@@ -1852,7 +1886,7 @@ __device__ __forceinline__ void limit_dot_lin_tile(const Geo<T> g, const T *cin,
   const int Kp = g.Kp;
   const bool staged = k0 < g.K;
   const int rD = 0, rQ = N, rC0 = NT - 2 * N, rC = rC0 + N;
-  const int vtIn = (int)StageRows<T, P>::bytes(NT, 1), vtOff = vt_on<T>() ? vtIn + 2 * g.vtMax * (int)sizeof(T) : -1;
+  const int vtIn = (int)StageRows<T, P>::bytes(NT, 1), vtOff = vt_on<T>(g, 1) ? vtIn + 2 * g.vtMax * (int)sizeof(T) : -1;
   if (staged) {
     if (t == 0) { mbar_init(bar, 1); mbar_fence_init(); }
     if (vtOff >= 0) vt_reset(g, 1, vtOff);

@@ -77,6 +77,15 @@ constexpr int op_parts(int p) { return p == 0 ? 1 : 2; }
 constexpr int op_exp_words(int p) { return 1 + (op_parts(p) * ((p + 1) * (p + 2) / 2) + 3 + 3) / 4; }
 constexpr int corr_exp_words(int p) { return 1 + (p * ((p + 1) * (p + 2) / 2) + 3) / 4; }
 
+// Whether a block of elements works with the table of its vertices (Geo::vtMax the longest list) rather than
+// with every element's own keys: always for one quantity; for the Taylor limiters' two to six where the
+// list is short, as in Morton order (81 to 130 vertices per 128 elements).  A long list is as many loads
+// and atomics as the elements' own, in shared memory that the kernel then lacks as L1.  80000
+// triangles, FP32, hierarchical limiter, per step without / with tables: Morton order p = 3 141 / 114 us,
+// p = 2 83 / 70; rows of the grid (250 vertices) p = 3 125 / 123, p = 2 75 / 79; random order (384)
+// p = 3 244 / 363, p = 2 154 / 222.
+__host__ __device__ constexpr bool use_block_tables(int nc, int vtMax) { return nc == 1 || vtMax <= 160; }
+
 // Static per-element data of one mesh (device pointers, SoA with stride Kp).
 template <typename T> struct Geo {
   int K, Kp, numV, Vp;

@@ -170,7 +170,7 @@ static cudaError_t copy_state(dgadv_handle *h, void *dst, const void *src, size_
 // Shared memory of `n` block-local vertex tables (extremes read, or keys gathered), after a kernel's
 // staged rows; with blocks of another size than kBlock the tables are not used.
 template <typename T> static size_t vt_bytes(const dgadv_handle *h, int n, int block = kBlock) {
-  return block == kBlock ? (size_t)n * 2 * h->nc * h->vtMax * sizeof(T) : 0;
+  return block == kBlock && use_block_tables(h->nc, h->vtMax) ? (size_t)n * 2 * h->nc * h->vtMax * sizeof(T) : 0;
 }
 // ... of a producer's key table (32-bit keys: vt_on), beside n tables of extremes
 template <typename T> static size_t vt_key_bytes(const dgadv_handle *h, int n, int block = kBlock) {
@@ -226,10 +226,16 @@ static cudaError_t set_smem_attributes() {
     set0((const void *)k_op_fused<T, P, 2, true>, SR::bytes(SR::op(2, true), 1));
     set0((const void *)k_op_fused<T, P, 2, false>, SR::bytes(SR::op(2, true), 1));
   }
-  set((const void *)k_limit_dot<T, P, 1>, SR::bytes(SR::limdot(), 1));
-  set((const void *)k_limit_dot<T, P, 2>, SR::bytes(SR::limdot(), 1));
-  set((const void *)k_limit<T, P, 1>, SR::bytes(SR::lim(), 1));
-  set((const void *)k_limit<T, P, 2>, SR::bytes(SR::lim(), 1));
+  set((const void *)k_limit_dot<T, P, 1, true>, SR::bytes(SR::limdot(), 1));
+  set((const void *)k_limit_dot<T, P, 2, true>, SR::bytes(SR::limdot(), 1));
+  set((const void *)k_limit<T, P, 1, true>, SR::bytes(SR::lim(), 1));
+  set((const void *)k_limit<T, P, 2, true>, SR::bytes(SR::lim(), 1));
+  if constexpr (P >= 2) {
+    set0((const void *)k_limit_dot<T, P, 1, false>, SR::bytes(SR::limdot(), 1));
+    set0((const void *)k_limit_dot<T, P, 2, false>, SR::bytes(SR::limdot(), 1));
+    set0((const void *)k_limit<T, P, 1, false>, SR::bytes(SR::lim(), 1));
+    set0((const void *)k_limit<T, P, 2, false>, SR::bytes(SR::lim(), 1));
+  }
   set0((const void *)k_to_taylor<T, P>, SR::bytes(SR::totaylor(), 0));
   if constexpr (std::is_same_v<T, float> && P >= 2) {
     set0((const void *)k_stage_op_mma<P, true>, MmaSmem<P>::bytes(true));
@@ -253,6 +259,20 @@ static auto stage_kernel(const dgadv_handle *h) -> decltype(&k_stage_op<T, P, MO
 template <typename T, int P>
 static int stage_rows(const dgadv_handle *h, int mode, bool lin, bool rhs) {
   return StageRows<T, P>::op(mode, lin, kHasElementOperator<T> && (!rhs || std::is_same_v<T, double>) && element_operator_on(h));
+}
+
+// The Taylor limiters' kernels, with or without the block's table of extremes.
+template <typename T, int P, int LT>
+static auto taylor_limdot(const dgadv_handle *h) -> decltype(&k_limit_dot<T, P, LT, true>) {
+  if constexpr (P >= 2)
+    if (!use_block_tables(h->nc, h->vtMax)) return &k_limit_dot<T, P, LT, false>;
+  return &k_limit_dot<T, P, LT, true>;
+}
+template <typename T, int P, int LT>
+static auto taylor_lim(const dgadv_handle *h) -> decltype(&k_limit<T, P, LT, true>) {
+  if constexpr (P >= 2)
+    if (!use_block_tables(h->nc, h->vtMax)) return &k_limit<T, P, LT, false>;
+  return &k_limit<T, P, LT, true>;
 }
 
 template <typename T, int P>
@@ -336,9 +356,9 @@ static cudaError_t launch_step(dgadv_handle *h, double t0, double tau) {
       prof_mark(h, 1);
       if (lin) launch_k(h, k_limit_dot_lin<T, P>, grid, SR::bytes(SR::limdot_lin_rows(h->mtOnTheFly), 1) + vt_key_bytes<T>(h, 1), g, (const T *)in, (const T *)cn, (const T *)cdB, yB, lim_in<T>(lo1, h), lo2, sc);
       else if (h->limType == DGADV_LIM_STRICT)
-        launch_k(h, k_limit_dot<T, P, 2>, grid, SR::bytes(SR::limdot(), 1) + vt_key_bytes<T>(h, 1), g, in, cn, (const T *)cdB, yB, lim_in<T>(lo1, h), lo2, sc);
+        launch_k(h, taylor_limdot<T, P, 2>(h), grid, SR::bytes(SR::limdot(), 1) + vt_key_bytes<T>(h, 1), g, in, cn, (const T *)cdB, yB, lim_in<T>(lo1, h), lo2, sc);
       else
-        launch_k(h, k_limit_dot<T, P, 1>, grid, SR::bytes(SR::limdot(), 1) + vt_key_bytes<T>(h, 1), g, in, cn, (const T *)cdB, yB, lim_in<T>(lo1, h), lo2, sc);
+        launch_k(h, taylor_limdot<T, P, 1>(h), grid, SR::bytes(SR::limdot(), 1) + vt_key_bytes<T>(h, 1), g, in, cn, (const T *)cdB, yB, lim_in<T>(lo1, h), lo2, sc);
       prof_mark(h, -1);
       loS = lo2;
     }
@@ -347,9 +367,9 @@ static cudaError_t launch_step(dgadv_handle *h, double t0, double tau) {
     prof_mark(h, 2);
     if (lin) launch_k(h, k_limit_lin<T, P>, gridK, vt_bytes<T>(h, 1), g, (const T *)yB, out, lim_in<T>(loS, h), scBC);
     else if (h->limType == DGADV_LIM_STRICT)
-      launch_k(h, k_limit<T, P, 2>, grid, SR::bytes(SR::lim(), 1) + vt_bytes<T>(h, 1), g, (const T *)yB, out, lim_in<T>(loS, h), scBC);
+      launch_k(h, taylor_lim<T, P, 2>(h), grid, SR::bytes(SR::lim(), 1) + vt_bytes<T>(h, 1), g, (const T *)yB, out, lim_in<T>(loS, h), scBC);
     else
-      launch_k(h, k_limit<T, P, 1>, grid, SR::bytes(SR::lim(), 1) + vt_bytes<T>(h, 1), g, (const T *)yB, out, lim_in<T>(loS, h), scBC);
+      launch_k(h, taylor_lim<T, P, 1>(h), grid, SR::bytes(SR::lim(), 1) + vt_bytes<T>(h, 1), g, (const T *)yB, out, lim_in<T>(loS, h), scBC);
     prof_mark(h, -1);
   }
   if (S == 1 && nRun == 1 && (const T *)dst == cn && !h->stepRecordsOnly) return copy_state(h, dst, cA, (size_t)h->N * h->Kp * sizeof(T));
@@ -437,9 +457,9 @@ static cudaError_t launch_limit_state(dgadv_handle *h, double t) {
   } else {
     launch_k(h, k_to_taylor<T, P>, grid, SR::bytes(SR::totaylor(), 0), g, (const T *)h->cn, (T *)h->tbuf, lo, sc);
     if (h->limType == DGADV_LIM_STRICT)
-      launch_k(h, k_limit<T, P, 2>, grid, SR::bytes(SR::lim(), 1) + vt_bytes<T>(h, 1), g, (const T *)h->tbuf, (T *)h->cn, lim_in<T>(lo, h), sc);
+      launch_k(h, taylor_lim<T, P, 2>(h), grid, SR::bytes(SR::lim(), 1) + vt_bytes<T>(h, 1), g, (const T *)h->tbuf, (T *)h->cn, lim_in<T>(lo, h), sc);
     else
-      launch_k(h, k_limit<T, P, 1>, grid, SR::bytes(SR::lim(), 1) + vt_bytes<T>(h, 1), g, (const T *)h->tbuf, (T *)h->cn, lim_in<T>(lo, h), sc);
+      launch_k(h, taylor_lim<T, P, 1>(h), grid, SR::bytes(SR::lim(), 1) + vt_bytes<T>(h, 1), g, (const T *)h->tbuf, (T *)h->cn, lim_in<T>(lo, h), sc);
   }
   return cudaGetLastError();
 }

@@ -198,6 +198,30 @@ def test_block_vertex_tables(lib, precision, p, lim):
     assert np.array_equal(out[0], out[1])
 
 
+# Lists between the two: the caller's rows (NO_REORDER), three vertex lines of 65 per 128 elements.  The
+# Taylor limiters then read every element's own keys, the library's own order has tables.
+@pytest.mark.parametrize('precision,p,lim', [('fp32', 2, 'hierarch_vert'), ('fp32', 3, 'strict'), ('df32', 2, 'strict'),
+                                             ('df32', 3, 'hierarch_vert'), ('fp64', 2, 'hierarch_vert'),
+                                             ('fp64', 3, 'strict')])
+def test_block_vertex_tables_in_row_order(lib, precision, p, lim):
+    from festung_gb300 import _lib as L
+    from festung_gb300.solver import DeviceSolver
+    coordV, V0T = mesh(64)
+    out = []
+    for flags in (0, L.FLAG_NO_REORDER):
+        s = DeviceSolver(coordV, V0T, p, min(p + 1, 3), precision=precision, isSlopeLim=True, typeSlopeLim=lim,
+                         flags=flags)
+        try:
+            s.set_velocity_function((L.VEL_ROTATION, []))
+            s.project_state((L.FN_GAUSS_SLOT, []), 0.0, 2 * p + 1)
+            s.limit_state(0.0)
+            s.step(3, 0, 1e-4)
+            out.append(s.get_state())
+        finally:
+            s.close()
+    assert np.array_equal(out[0], out[1])
+
+
 # Species share their launches; each must come out as if it ran alone, also on a handle whose
 # buffers an earlier, larger set of species left behind.
 @pytest.mark.parametrize('precision', ['fp64', 'fp32'])
