@@ -55,18 +55,15 @@ template <int P> const void *fx_symbol();                // ... of the FP64 unit
   template <> [[maybe_unused]] const void *tab_symbol<T, 3>() { return (const void *)&NAME##3; }  \
   }
 
-// The digit tables of the FP64 units (dgadv_fixed.cuh).
+// The digit tables of the FP64 units (dgadv_fixed.cuh), degrees 1 to 3.
 #define DGADV_DEFINE_DIGIT_TABLES(NAME)                                                         \
-  static __constant__ FxTab<0> NAME##0;                                                         \
   static __constant__ FxTab<1> NAME##1;                                                         \
   static __constant__ FxTab<2> NAME##2;                                                         \
   static __constant__ FxTab<3> NAME##3;                                                         \
-  template <> __device__ __forceinline__ const FxTab<0> &fx_tab<0>() { return NAME##0; }        \
   template <> __device__ __forceinline__ const FxTab<1> &fx_tab<1>() { return NAME##1; }        \
   template <> __device__ __forceinline__ const FxTab<2> &fx_tab<2>() { return NAME##2; }        \
   template <> __device__ __forceinline__ const FxTab<3> &fx_tab<3>() { return NAME##3; }        \
   namespace {                                                                                   \
-  template <> [[maybe_unused]] const void *fx_symbol<0>() { return (const void *)&NAME##0; }    \
   template <> [[maybe_unused]] const void *fx_symbol<1>() { return (const void *)&NAME##1; }    \
   template <> [[maybe_unused]] const void *fx_symbol<2>() { return (const void *)&NAME##2; }    \
   template <> [[maybe_unused]] const void *fx_symbol<3>() { return (const void *)&NAME##3; }    \
@@ -1145,10 +1142,15 @@ __device__ __forceinline__ void stage_op_tile(const Geo<T> g, const T *cin, cons
            const LimOut<T> lo, const StageScalars sc, const int tile, const int nTiles = -1) {
   constexpr int N = Dims<P>::N, Q = Dims<P>::Q, R = Dims<P>::R, NQ = NCQ<P>::value;
   constexpr bool OPF = VAR == kOpFp32, EOP = VAR == kOpElement;
-  constexpr bool FXP = EOP && std::is_same_v<T, double>;   // the element operator in fixed point
+  constexpr bool E64 = EOP && std::is_same_v<T, double>;   // source terms, if any, with hatM^-1 applied
+  constexpr bool FXP = E64 && P >= 1;                      // ... its sums in fixed point (p = 0: single products)
   static_assert(!EOP || ((std::is_same_v<T, double> || std::is_same_v<T, df32>) && !RHS),
                 "the element operator is FP64 or double-float without source terms");
   using A = std::conditional_t<OPF, float, T>;
+  // The fixed-point form has the longer chain: on a mesh of a few blocks, without a limiter, the nine products
+  // of p = 1 are done sooner in FP64 (128 triangles 7.9 us per step, 9.1 in fixed point; 2048: 8.7 and 9.0; 80000:
+  // 40 and 20).
+  [[maybe_unused]] const bool digits = FXP && g.AopX && !(P == 1 && MODE == 0 && g.K <= 16 * kBlock);
   // with the mass solve (FP64, double-float) and no source terms, hatM^-1 is folded into the
   // test-function tables of the volume and flux terms (Fg1, Fg2, Fphi)
   constexpr bool kFold = sizeof(A) == 8 && !RHS;
@@ -1175,7 +1177,7 @@ __device__ __forceinline__ void stage_op_tile(const Geo<T> g, const T *cin, cons
     __syncthreads();
     if (t == 0) {                                 // static rows before the dependency wait
       stage_expect<T>(bar, NT - (MODE != 2 && first ? N : 0), 1);
-      if (FXP && g.AopX) {       // digits: 8 bytes each, as the rows they stand for
+      if (digits) {              // 8 bytes each, as the rows they stand for
         stage_T(smem, rF, (const T *)g.AopX, N * N, Kp, k0, bar);
         stage_T(smem, rV, (const T *)g.VnX, 3 * R, Kp, k0, bar);
       } else {
@@ -1195,10 +1197,9 @@ __device__ __forceinline__ void stage_op_tile(const Geo<T> g, const T *cin, cons
   if (MODE != 0 && active) load_vertices(g, k, vt, vid);
   VtList vl{0, 0, 0};
   if (vt && staged) vl = vt_list(g, tile);
-  fx::OpExp<P> ax;
-  T src[N];                                       // the source terms at this stage's time
-  if constexpr (FXP) {                            // neighbours across inflow edges only
-    if (active && g.aopE) ax.load(g.aopE, Kp, k);
+  [[maybe_unused]] fx::OpExp<P> ax;
+  [[maybe_unused]] T src[N];                      // the source terms at this stage's time
+  if constexpr (E64)
     if (g.rhsM) {
 #pragma unroll
       for (int i = 0; i < N; ++i) src[i] = T(0);
@@ -1208,10 +1209,13 @@ __device__ __forceinline__ void stage_op_tile(const Geo<T> g, const T *cin, cons
         for (int i = 0; i < N; ++i) src[i] += gm * g.rhsM[((size_t)m * N + i) * Kp + k];
       }
     }
+  if constexpr (FXP)                              // neighbours across inflow edges only
+    if (active && digits) {
+      ax.load(g.aopE, Kp, k);
 #pragma unroll
-    for (int n = 0; n < 3; ++n)
-      if (active && g.aopE && !ax.inflow(n)) nb[n] = -1;
-  }
+      for (int n = 0; n < 3; ++n)
+        if (!ax.inflow(n)) nb[n] = -1;
+    }
   pdl_wait();
   pdl_trigger();
   if (MODE != 0) reset_next<T>(g, lo, k, nTiles < 0 ? -1 : tile, nTiles);
@@ -1267,7 +1271,7 @@ __device__ __forceinline__ void stage_op_tile(const Geo<T> g, const T *cin, cons
       for (int i = 0; i < N; ++i)
 #pragma unroll
         for (int j = 0; j < N; ++j)
-          rhs[i].fma(FXP ? g.Aop[(size_t)(i * N + j) * Kp + k] : srow<T>(smem, rF + i * N + j)[t], c[j]);
+          rhs[i].fma(digits ? g.Aop[(size_t)(i * N + j) * Kp + k] : srow<T>(smem, rF + i * N + j)[t], c[j]);
     } else {
     // volume term (at p = 3, 12 points: unrolled by 3 to keep the body in the instruction cache)
 #pragma unroll(P >= 3 ? 3 : Q)
@@ -1328,7 +1332,7 @@ __device__ __forceinline__ void stage_op_tile(const Geo<T> g, const T *cin, cons
       }
 #pragma unroll
       for (int r2 = 0; r2 < R; ++r2) {
-        const A v = as_arith<A>(FXP ? g.Vn[(size_t)(n * R + r2) * Kp + k] : srow<T>(smem, rV + n * R + r2)[t]);
+        const A v = as_arith<A>(digits ? g.Vn[(size_t)(n * R + r2) * Kp + k] : srow<T>(smem, rV + n * R + r2)[t]);
         if (EOP && !(v < A(0) && nb[n] >= 0)) continue;
         Acc<A> tr(A(0));
         if (v > A(0) && outOk) {
@@ -1361,7 +1365,7 @@ __device__ __forceinline__ void stage_op_tile(const Geo<T> g, const T *cin, cons
       for (int i = 0; i < N; ++i) cdot[i] = T(rhs[i].get());
     }
     }
-    if constexpr (FXP)
+    if constexpr (E64)
       if (g.rhsM)
 #pragma unroll
         for (int i = 0; i < N; ++i) cdot[i] += src[i];

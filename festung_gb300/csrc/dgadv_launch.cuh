@@ -10,7 +10,7 @@
 
 namespace dgadv {
 
-template <typename T, int P, bool DIGITS = std::is_same_v<T, double>>
+template <typename T, int P, bool DIGITS = std::is_same_v<T, double> && P >= 1>
 static cudaError_t upload_tables(const RefTables &rt) {
   Tab<T, P> t;
   fill_tables(rt, t);
@@ -574,7 +574,6 @@ static cudaError_t dispatch_build_element_operator(dgadv_handle *h) {
                                                           h->nbr, (Dig *)h->AopX, (Dig *)h->VnX, h->aopE);
       };
       switch (h->p) {
-        case 0: fix(std::integral_constant<int, 0>()); break;
         case 1: fix(std::integral_constant<int, 1>()); break;
         case 2: fix(std::integral_constant<int, 2>()); break;
         case 3: fix(std::integral_constant<int, 3>()); break;

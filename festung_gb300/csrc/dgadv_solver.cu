@@ -787,7 +787,9 @@ int dgadv::refresh_element_operator(dgadv_handle *h) {
     int st;
     if ((st = dev_alloc(h, &h->Aop, (size_t)h->N * h->N * h->Kp * o.realBytes))) return st;
     DG_CUDA(cudaMemset(h->Aop, 0, (size_t)h->N * h->N * h->Kp * o.realBytes));
-    if (h->prec == DGADV_FP64)   // its digits, where there is room: without them the sums run in FP64
+    // its digits, where there is room (without them the sums run in FP64, as at p = 0: 128 triangles 3.1 us
+    // per step so, 3.9 in fixed point)
+    if (h->prec == DGADV_FP64 && h->p >= 1)
       alloc_optional(h, {{&h->AopX, (size_t)h->N * h->N * h->Kp * 8}, {&h->VnX, (size_t)3 * h->R * h->Kp * 8},
                          {(void **)&h->aopE, (size_t)op_exp_words(h->p) * h->Kp * 4}});
   }
