@@ -53,6 +53,8 @@ template <int W> __device__ __forceinline__ long long fix(double x, int E) {
   const long long v = (long long)fix_mag<W>(x, E), sg = (long long)(__double2hiint(x) >> 31);
   return (v ^ sg) - sg;
 }
+// x in the same units to the nearest (halves up).
+template <int W> __device__ __forceinline__ long long fix_near(double x, int E) { return (fix<W + 1>(x, E) + 1) >> 1; }
 // X = h 2^31 + l, -2^30 <= l < 2^30
 __host__ __device__ __forceinline__ Dig digits(long long X) {
   Dig d;

@@ -271,9 +271,9 @@ struct GridSums {
   unsigned int *ticket;     // blocks that have stored their shares (0 between launches)
   double *out;
 };
-// Sums x[0 .. n) over a warp's lanes, in every lane.  On the integer units: each share scaled to 57 bits
-// below the lanes' largest exponent (off by at most 2^-57 of it, where an FP64 addition rounds at
-// 2^-53), one redux and five exchanges and additions of 64-bit words, n sums side by side; five FP64
+// Sums x[0 .. n) over a warp's lanes, in every lane.  On the integer units: each share rounded to 57 bits
+// below the lanes' largest exponent (off by at most 2^-58 of it, and no share one way, where each FP64
+// addition rounds at 2^-53), one redux and five exchanges and additions of 64-bit words, n sums side by side; five FP64
 // additions each would hold the warp's scheduler for 380 cycles.  Shares outside 2^(+-800) take the
 // FP64 form.
 template <int n> __device__ __forceinline__ void warp_sums(double x[n]) {
@@ -293,7 +293,7 @@ template <int n> __device__ __forceinline__ void warp_sums(double x[n]) {
   }
   long long v[n];
 #pragma unroll
-  for (int q = 0; q < n; ++q) v[q] = fx::fix<57>(x[q], max(E[q], 223));   // all zero: zero
+  for (int q = 0; q < n; ++q) v[q] = fx::fix_near<57>(x[q], max(E[q], 223));   // all zero: zero
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1)
 #pragma unroll

@@ -263,3 +263,14 @@ extern "C" int fixed_point_limiter(int p, int numV, const double *coordV, int nu
   if (!build_grid(numV, coordV, numT, V0T, gr, err)) return 1;
   return p == 2 ? run_limiter<2>(gr, solution != 0, c, o) : run_limiter<3>(gr, solution != 0, c, o);
 }
+
+// The sum of each 32 of x as the implicit solver's warps form it (57 bits below the largest exponent).
+extern "C" void fixed_point_lane_sums(int n, const double *x, double *out) {
+  for (int i = 0; i < n; ++i) {
+    int E = 223;
+    long long v = 0;
+    for (int l = 0; l < 32; ++l) E = std::max(E, fx::expo(x[32 * i + l]));
+    for (int l = 0; l < 32; ++l) v += fx::fix_near<57>(x[32 * i + l], E);
+    out[i] = fx::to_double_int(v, E - 1022 - 57);
+  }
+}

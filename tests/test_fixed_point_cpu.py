@@ -194,3 +194,20 @@ def test_limiter_of_small_states(host, p, solution, e):
     r = call(host.fixed_point_limiter, m, p, solution, c)
     assert np.all(r.taken) or e < -690 or solution   # (a tiny slope times a tiny factor is handed back too)
     close(r, 16)
+
+
+# Sums over a warp's lanes: shares alike, of one sign, decades apart, one far above the rest.
+@pytest.mark.parametrize('data', ['normal', 'squares', 'decades', 'one'])
+def test_lane_sums_are_no_less_accurate_than_fp64(host, data):
+    r = np.random.default_rng(1)
+    x = {'normal': r.standard_normal, 'squares': lambda s: r.standard_normal(s) ** 2,
+         'decades': lambda s: np.exp(10 * r.standard_normal(s)),
+         'one': lambda s: r.random(s) * np.where(np.arange(32) == 0, 1.0, 1e-6)}[data]((20000, 32))
+    out = np.zeros(len(x))
+    host.fixed_point_lane_sums(len(x), np.ascontiguousarray(x).ctypes.data_as(C.c_void_p),
+                               out.ctypes.data_as(C.c_void_p))
+    tree, exact = x, x.astype(np.longdouble).sum(axis=1)
+    while tree.shape[1] > 1:
+        tree = tree[:, :tree.shape[1] // 2] + tree[:, tree.shape[1] // 2:]
+    size = np.abs(x).sum(axis=1)
+    assert rms((out - exact) / size) <= rms((tree[:, 0] - exact) / size)
