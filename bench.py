@@ -853,6 +853,43 @@ def side_path(wl, precision, device, c0, flush, reps, options=None):
             'kernels': kern, 'roofline': roof, 'whole_stage': whole_stage_roofline(pd, w, ms)}, c
 
 
+HEADLINE = ('metric', 'value', 'unit', 'n_gpus', 'steps', 'warmup', 'ms_per_step', 'ms_per_step_unit',
+            'higher_is_better', 'scaling', 'vs_baseline', 'dtype', 'data', 'config', 'clocks', 'e2e', 'gpu_launches',
+            'cpu_baseline')
+
+
+def headline(result):
+    """The line for stdout: the headline's own entries, its roofline and kernel times, and one number
+    (`value`, or its unit's own key) per side workload.  The full record of every block, some 20 KB, is
+    `--details FILE`, or a line on stderr."""
+    def short(x):
+        return float('%.4g' % x) if isinstance(x, float) else x
+
+    line = {k: result[k] for k in HEADLINE if k in result}
+    roof = result['roofline']
+    line['roofline'] = {k: short(roof[k]) for k in ('bound', 'kernel', 'achieved', 'peak', 'unit', 'frac', 'traffic')
+                        if k in roof}
+    line['kernels_ms'] = {k: short(v['ms_per_launch_live']) for k, v in result['kernels'].items()}
+    line['whole_stage_frac'] = short(result['whole_stage']['frac'])
+    side = {}
+
+    def collect(name, block):
+        if not isinstance(block, dict):
+            return
+        for key in ('value', 'ms_per_step', 'backward_over_forward'):
+            if isinstance(block.get(key), (int, float)):
+                side[name] = short(float(block[key]))
+                break
+        for k, v in block.items():
+            if k not in ('kernels', 'roofline', 'whole_stage', 'launch', 'paths'):
+                collect('%s.%s' % (name, k), v)
+    for k, v in result.items():
+        if k not in line and k not in ('kernels', 'whole_stage'):
+            collect(k, v)
+    line['side'] = dict(sorted(side.items())[:48])
+    return line
+
+
 def run_ours(args):
     rank, world, local = dist_env()
     device = local
@@ -1022,7 +1059,12 @@ def run_ours(args):
                       'assembly as the reference; scipy sparse is single-threaded), %.1f s on a %d-core host'
                       % (args.cpu_stages, dt, n)}
     if rank == 0:
-        print(json.dumps(result), flush=True)
+        if args.details:
+            with open(args.details, 'w') as f:
+                json.dump(result, f, indent=1)
+        else:
+            print('details: ' + json.dumps(result), file=sys.stderr, flush=True)
+        print(json.dumps(headline(result)), flush=True)
     if world > 1:
         torch.distributed.destroy_process_group()
     return 0
@@ -1045,6 +1087,7 @@ def main():
     ap.add_argument('--no-large', action='store_true')
     ap.add_argument('--no-transport', action='store_true')
     ap.add_argument('--no-cpu', action='store_true')
+    ap.add_argument('--details', default=None, help='file for the full record (default: a line on stderr)')
     ap.add_argument('--cpu-stages', type=int, default=1)
     ap.add_argument('--ref-stages-per-step', type=int, default=1)
     ap.add_argument('--ncu-case', default=None, choices=sorted(WORKLOADS) + ['adjoint', 'implicit', 'transport'],
