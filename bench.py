@@ -258,17 +258,14 @@ def run_reference(args):
     return 0
 
 
-# DRAM bytes per launch (dram__bytes_read.sum + dram__bytes_write.sum) of the stage kernels,
-# from single-kernel ncu captures (-k <kernel> -c 1, cold L2 under ncu) of
-# `bench.py --ncu-case <workload> --precision <p> --ncu-steps 2`, keyed (workload, precision,
-# kernel).
-# FP64 floating-point operations per element of the FP64 stage kernels (2 x DFMA + DADD + DMUL
-# thread instructions, smsp__sass_thread_inst_executed_op_{dfma,dadd,dmul}_pred_on.sum of one
-# single-kernel ncu capture each, divided by the elements), keyed (workload, kernel):
-# profiles/stage_kernels_131k_fp64_full.md.
-MEASURED_FP64_FLOPS = {('gauss_slot_131k_p2', 'k_stage_op'): 197.1,
-                       ('gauss_slot_131k_p2', 'k_limit_dot'): 192.4,
-                       ('gauss_slot_131k_p2', 'k_limit'): 117.5}
+# FP64 floating-point operations per element that the FP64 stage kernels execute (2 x DFMA + DADD +
+# DMUL thread instructions, smsp__sass_thread_inst_executed_op_{dfma,dadd,dmul}_pred_on.sum of one
+# ncu capture, third stage, divided by the elements), keyed (workload, kernel):
+# profiles/stage_kernels_131k_fp64_full.md.  Most sums run in fixed point on the integer units and
+# count nothing here.
+MEASURED_FP64_FLOPS = {('gauss_slot_131k_p2', 'k_stage_op'): 26.0,
+                       ('gauss_slot_131k_p2', 'k_limit_dot'): 76.6,
+                       ('gauss_slot_131k_p2', 'k_limit'): 25.8}
 
 
 def fp64_peak(reps=5, n=4096):
@@ -291,13 +288,16 @@ def fp64_peak(reps=5, n=4096):
     return 2.0 * n ** 3 / (best * 1e-3) / 1e12
 
 
-MEASURED_TRAFFIC = {('gauss_slot_131k_p2', 'fp32', 'k_stage_op'): 18.4e6,
-                    ('gauss_slot_131k_p2', 'fp32', 'k_limit_dot'): 28.4e6,
-                    ('gauss_slot_131k_p2', 'fp32', 'k_limit'): 5.8e6,
-                    # FP64, element operator on (ncu, one cold launch each; dram read + write)
-                    ('gauss_slot_131k_p2', 'fp64', 'k_stage_op'): 58.5e6,
-                    ('gauss_slot_131k_p2', 'fp64', 'k_limit_dot'): 54.8e6,
-                    ('gauss_slot_131k_p2', 'fp64', 'k_limit'): 9.5e6}
+# DRAM bytes per launch (dram__bytes_read.sum + dram__bytes_write.sum) of the stage kernels, third
+# stage, cold L2 under ncu, of `bench.py --ncu-case <workload> --precision <p> --ncu-steps 2`, keyed
+# (workload, precision, kernel).  FP32 with the correction rebuilt from B; FP64 with the element
+# operator's and the correction's digits.
+MEASURED_TRAFFIC = {('gauss_slot_131k_p2', 'fp32', 'k_stage_op'): 17.9e6,
+                    ('gauss_slot_131k_p2', 'fp32', 'k_limit_dot'): 14.3e6,
+                    ('gauss_slot_131k_p2', 'fp32', 'k_limit'): 5.3e6,
+                    ('gauss_slot_131k_p2', 'fp64', 'k_stage_op'): 61.5e6,
+                    ('gauss_slot_131k_p2', 'fp64', 'k_limit_dot'): 58.0e6,
+                    ('gauss_slot_131k_p2', 'fp64', 'k_limit'): 9.1e6}
 
 
 def large_block(device, flush):
@@ -808,7 +808,7 @@ def whole_stage_roofline(pd, w, ms_per_solve):
 
 
 def hbm_block(device, flush, reps=2):
-    """The HBM-bound case of the p = 2 operator: the 131072-triangle workload's operator and
+    """The p = 2 operator with inputs from HBM: the 131072-triangle workload's operator and
     limiter on a 16x larger mesh (2,097,152 triangles, FP32 working set ~0.5 GB, far beyond
     L2), 500 steps from c0: the whole stage against the scope table's bytes, and each kernel."""
     pd = setup_problem('gauss_slot_2M_p2', 'fp32', device)
@@ -939,12 +939,13 @@ def run_ours(args):
     value = world * units / (ms_per_step / 1e3)
     kern, roof = kernel_table(s, pd, 8, ms_per_step)
     roof['traffic'] = MEASURED_TRAFFIC.get((wl, 'fp64', roof['kernel']))
-    roof['note'] = ('L2-resident: the bytes a FP64 stage touches on this mesh (about 120 MB cold per '
+    roof['note'] = ('L2-resident: the bytes a FP64 stage touches on this mesh (about 129 MB cold per '
                     'stage with the element operator, traffic) fit the 129 MB L2 for the most part, so '
                     'they are served mostly from L2 once a solve runs; the FP64 kernels are bound '
-                    'by instruction issue and latency, not by bandwidth (their sums run in fixed point on '
-                    'the integer units, fp64_rate); the HBM-bound figure is hbm_case')
-    # the FP64 operations they stand for, against cuBLAS DGEMM on the same GPU
+                    'by instruction issue and latency, not by bandwidth: most of their sums run in fixed '
+                    'point on the integer units, and fp64_rate counts the FP64 operations that are left; '
+                    'the case with inputs beyond L2 is hbm_case')
+    # the FP64 operations the kernels execute, against cuBLAS DGEMM on the same GPU
     peak64 = fp64_peak()
     rate = {'peak_tflops': peak64, 'peak_source': 'measured: cuBLAS DGEMM 4096^3 (torch.matmul float64)',
             'kernels': {}}

@@ -28,3 +28,19 @@ def test_the_line_is_short_and_complete():
     assert line['side']['ensemble.groups.1'] == 5.0e10
     assert line['side']['adjoint.fp32.snapshots_20'] == 2.5
     assert len(json.dumps(line)) < 4000 < len(json.dumps(result))
+
+
+def test_the_rates_divide_the_present_kernels_counters():
+    """FP64 operations and DRAM bytes per launch are constants: they have to be the ones of the counter
+    summary of the kernels in the tree, not of kernels that these replaced."""
+    import bench
+    path = os.path.join(os.path.dirname(bench.__file__), 'profiles', 'stage_kernels_131k_fp64_full.md')
+    present = open(path).read().split('## The FP64 forms before')[0]
+    row = {r[1].strip(): [c.strip() for c in r[2:-1]] for r in (x.split('|') for x in present.splitlines()) if len(r) == 6}
+    names = ('k_stage_op', 'k_limit_dot', 'k_limit')
+    per = [[float(x) for x in row[k + ' / element']] for k in ('DFMA', 'DADD', 'DMUL')]
+    for i, name in enumerate(names):
+        flops = bench.MEASURED_FP64_FLOPS[('gauss_slot_131k_p2', name)]
+        assert flops == float(row['FP64 flops / element (2 DFMA + DADD + DMUL)'][i])
+        assert abs(flops - (2 * per[0][i] + per[1][i] + per[2][i])) <= 0.25      # four roundings of 0.05
+        assert bench.MEASURED_TRAFFIC[('gauss_slot_131k_p2', 'fp64', name)] == float(row['DRAM read + write (MB)'][i]) * 1e6
