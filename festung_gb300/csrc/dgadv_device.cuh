@@ -707,7 +707,7 @@ __device__ __forceinline__ void stage_expect(uint64_t *bar, int nT, int nI) {
 // kernels piles up on the SMs, each placed where the ones before it left room: their blocks end up
 // on few SMs, and a chain can run slower than without the early launch (four species on 8192
 // triangles, p = 1, FP64: 123 us per step so, 50 us now; 6498 triangles, p = 2, FP64: 45 and 23.5 us
-// per stage, 30 without dependent launch).
+// per stage with the later trigger, 30 without dependent launch).
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 // A kernel in such a chain must not declare a buffer that earlier kernels of the chain write as
@@ -1133,7 +1133,8 @@ __host__ __device__ constexpr bool basis_in_x1(int i) { return i == 0 || i == 1 
 //               terms are evaluated at the edge points, of neighbours that only inflow edges load.
 //               In FP64 the sums run in fixed point on the integer units (dgadv_fixed.cuh), since
 //               GB300's FP64 rate bounds them otherwise: 131072 triangles, p = 2, per launch (cold)
-//               51 -> 27 us, 2180 instructions per warp of which 20 in FP64 (about 190 before).
+//               52 -> 34 us, 2490 instructions per warp of which 26 in FP64 (101 before); what is left is
+//               latency, at four warps per scheduler (128 registers).
 //               Source terms are added in FP64, with hatM^-1 applied when they are set.
 constexpr int kOpPlain = 0, kOpFp32 = 1, kOpElement = 2;
 

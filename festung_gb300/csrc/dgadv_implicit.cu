@@ -30,7 +30,8 @@ namespace {
 constexpr int kImplBlock = 128;
 // Every kernel over the elements runs blocks of 32 elements x N coefficient rows, a warp per row: FP64
 // instructions issue at their full (low) rate only with warps on all four schedulers of an SM, and
-// the reference's 8192 elements are 256 warps with a thread per element, under two per SM.
+// the reference's 8192 elements are 256 warps with a thread per element, under two per SM.  Larger meshes do
+// not lose by it: 524288 elements, p = 1, 567 us per iteration with a thread per element, 397 so.
 constexpr int kRows = 32;             // elements per block
 constexpr int kVecs = 8;              // basis vectors a thread has in flight at once
 constexpr int kCheck = 4;             // Arnoldi steps between two looks at the residual estimate
@@ -413,15 +414,16 @@ struct GmresDense {
 };
 
 // One Arnoldi step is three kernels over the elements (it was eleven launches and 90 us at 8192
-// elements, p = 2; now 45 us):
+// elements, p = 2; now about 40 us):
 //   k_arn_apply   w = A P^-1 v_j; h1 = V^T w.  z = P^-1 v_j comes from the step before.  P inverts the
 //                 element's own block of A, so the local part of A z is v_j itself and only the
 //                 neighbours' inflow is left (IDENT; a mesh with a block whose stored inverse is off, or
 //                 singular with the identity in its place, applies the whole operator)
 //   k_arn_first   w -= V h1; h2 = V^T w and |w|^2        (classical Gram-Schmidt, second pass)
 //   k_arn_second  w -= V h2; v_{j+1} = w / |w|, with |w|^2 after the pass from |w|^2 - |h2|^2 (h2 is at
-//                 rounding level: no cancellation); z = P^-1 v_{j+1}; column j of the Hessenberg matrix and
-//                 the Givens rotations in one more block
+//                 rounding level beside w, until the Krylov space is used up and the residual is there too);
+//                 z = P^-1 v_{j+1}; column j of the Hessenberg matrix and the Givens rotations in one more
+//                 block
 template <typename T, int P, bool IDENT>
 __global__ void __launch_bounds__(kRows * IDims<P>::N)
 k_arn_apply(const ImplArgs<T> a, const T *__restrict__ V, size_t n, int j, const T *__restrict__ z, T *__restrict__ w,

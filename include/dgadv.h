@@ -105,6 +105,10 @@ enum {
                                    rebuilt whenever the velocity changes), which takes the FP64
                                    operator from about 244 to about 100 arithmetic instructions
                                    per element at p = 2; 0: evaluated at the quadrature points.
+                                   FP64 handles also keep these rows and the limiter's as integer
+                                   digits (p = 2, linear limiter: 636 bytes per element; p = 3:
+                                   1.7 KB); where the device has no room for them they are left
+                                   out and the sums run in FP64.
                                    The results agree to roundoff                              */
   DGADV_OPT_ADJ_GRAPH = 11      /* the reverse sweep captured as one CUDA graph (1) or launched
                                    directly (0); -1 (default): 1 without the limiter, 0 with it.
